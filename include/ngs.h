@@ -149,6 +149,19 @@ int ngs_knn_sdf(ngs_grid g, const int64_t* start, const int32_t* sorted, const f
                 const float* queries, int64_t nq, float inv_h, float h, int k, float stdv, int32_t* idx_out,
                 float* d2_out, float* sdf_out, ngs_stream s);
 
+/* The same queries through a tree of bounding boxes (32 points to a leaf, 32 children to a node): no
+ * cell size to choose and no cost for the empty space between a query and the points.  build orders
+ * the points and forms the boxes in `tree` (ngs_knn_tree_bytes(n), 16-byte aligned, kept by the caller
+ * for its queries); `scratch` (ngs_knn_tree_scratch_bytes(n)) is free again when the build has run.
+ * Results as ngs_knn_sdf's. */
+size_t ngs_knn_tree_bytes(int64_t n);
+size_t ngs_knn_tree_scratch_bytes(int64_t n);
+int ngs_knn_tree_build(const float* xyz, int64_t n, void* tree, size_t tree_bytes, void* scratch, size_t scratch_bytes,
+                       ngs_stream s);
+int ngs_knn_tree_query(const void* tree, size_t tree_bytes, const float* ref_xyz, int64_t n, const float* ref_normal,
+                       const float* queries, int64_t nq, int k, float stdv, int32_t* idx_out, float* d2_out,
+                       float* sdf_out, ngs_stream s);
+
 /* min/max of a float [n,3] array -> bbox_dev float[6] = (min xyz, max xyz) */
 int ngs_points_bbox(const float* xyz, int64_t n, float* bbox_dev, ngs_stream s);
 /* Mark the 8 trilinear corner cells of every point with level <= max_level

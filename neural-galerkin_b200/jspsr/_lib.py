@@ -96,6 +96,10 @@ _SIGS = {
     "ngs_knn_bucket": ([G, vp, i64, f32, vp, vp, vp], C.c_int),
     "ngs_knn_scatter": ([vp, i64, vp, vp, vp, vp], C.c_int),
     "ngs_knn_sdf": ([G, vp, vp, vp, vp, vp, i64, f32, f32, C.c_int, f32, vp, vp, vp, vp], C.c_int),
+    "ngs_knn_tree_bytes": ([i64], sz),
+    "ngs_knn_tree_scratch_bytes": ([i64], sz),
+    "ngs_knn_tree_build": ([vp, i64, vp, sz, vp, sz, vp], C.c_int),
+    "ngs_knn_tree_query": ([vp, sz, vp, i64, vp, vp, i64, C.c_int, f32, vp, vp, vp, vp], C.c_int),
     "ngs_splat_weights": ([G, vp, i64, f32, f64, vp, vp], C.c_int),
     "ngs_density_eval": ([G, vp, i64, f32, f64, vp, f32, C.c_int, vp, vp, vp, vp], C.c_int),
     "ngs_splat_data": ([G, vp, i64, f32, f64, vp, C.c_int, vp, vp, C.c_int, f32, vp, vp], C.c_int),

@@ -3,22 +3,20 @@
 Drop-in for the reference's ``ext.sdf_from_points(queries, ref_xyz, ref_normal, nb_points, stdv)``
 (``ext/__init__.py:11-16``, ``ext/sdfgen/sdf_from_points.cu:70-116``), the ground truth of the
 training loop (``models/full_net.py:135-142``).  The reference builds a CUDA k-d tree per call; here
-the reference points are bucketed on a uniform cell grid (a libngs rank bitmap of the occupied cells
-and a counting sort) and one kernel per query walks rings of cells until its k nearest points are
-final, then votes the sign (``csrc/knn.cu``).
+the reference points are ordered along a Morton curve by a counting sort and boxed 32 to a leaf in a
+32-ary tree, and one warp per query visits the boxes nearest first until no other can hold one of its
+k nearest points, then votes the sign (``csrc/knn.cu``).
 """
 from __future__ import annotations
 
-import math
-
-import numpy as np
 import torch
 
 from . import _lib as L
 
 
 class PointIndex:
-    """Reference points bucketed by cell for repeated nearest-neighbour queries."""
+    """Reference points in a box tree for repeated nearest-neighbour queries.  ``cell``, the cell size of
+    a grid index, has no effect: the tree sizes itself."""
 
     def __init__(self, ref_xyz: torch.Tensor, ref_normal: torch.Tensor = None, cell: float = None):
         L.require_cuda(ref_xyz, "ref_xyz")
@@ -27,31 +25,11 @@ class PointIndex:
         n = self.xyz.shape[0]
         if n == 0:
             raise ValueError("no reference points")
-        dev = self.xyz.device
-        lo, hi = self.xyz.min(0).values, self.xyz.max(0).values
-        ext = float((hi - lo).max().clamp(min=1e-6))
-        if cell is None:
-            # about 16 points per occupied cell for points on a surface (occupied cells ~ area / h^2)
-            cell = 4.0 * ext / math.sqrt(n)
-        cell = max(cell, ext / 1024.0)
-        self.h = float(cell)
-        self.inv_h = np.float32(1.0 / self.h)
-        clo = torch.floor(lo * self.inv_h).cpu().numpy().astype(np.int64)
-        chi = torch.floor(hi * self.inv_h).cpu().numpy().astype(np.int64)
-        self.grid, self.words = L.make_grid(clo, chi - clo + 1, 1, dev)
-        st = L.stream()
-        L.call("ngs_knn_mark_cells", self.grid, L.ptr(self.xyz), n, self.inv_h, st)
-        ncell = torch.empty(1, dtype=torch.int64, device=dev)
-        self._ws = L.grid_finalize(self.grid, self.words, ncell)
-        nc = int(ncell.item())
-        cell_of = torch.empty(n, dtype=torch.int32, device=dev)
-        count = torch.zeros(nc, dtype=torch.int32, device=dev)
-        L.call("ngs_knn_bucket", self.grid, L.ptr(self.xyz), n, self.inv_h, L.ptr(cell_of), L.ptr(count), st)
-        self.start = torch.empty(nc + 1, dtype=torch.int64, device=dev)
-        L.scan(count, out=self.start[:nc], total=self.start[nc:])
-        cursor = torch.zeros(nc, dtype=torch.int32, device=dev)
-        self.sorted = torch.empty(n, dtype=torch.int32, device=dev)
-        L.call("ngs_knn_scatter", L.ptr(cell_of), n, L.ptr(self.start), L.ptr(cursor), L.ptr(self.sorted), st)
+        lib, dev = L.load(), self.xyz.device
+        self.tree = torch.empty(lib.ngs_knn_tree_bytes(n), dtype=torch.uint8, device=dev)
+        scratch = torch.empty(lib.ngs_knn_tree_scratch_bytes(n), dtype=torch.uint8, device=dev)
+        L.call("ngs_knn_tree_build", L.ptr(self.xyz), n, L.ptr(self.tree), self.tree.numel(), L.ptr(scratch),
+               scratch.numel(), L.stream())
 
     def query(self, queries: torch.Tensor, k: int, stdv: float = None, want_knn: bool = True):
         """(indices int32 [Q, k], squared distances [Q, k], signed distance [Q] or None)."""
@@ -65,9 +43,9 @@ class PointIndex:
             if self.normal is None:
                 raise ValueError("signed distances need the reference normals")
             sdf = torch.empty(nq, dtype=torch.float32, device=dev)
-        L.call("ngs_knn_sdf", self.grid, L.ptr(self.start), L.ptr(self.sorted), L.ptr(self.xyz), L.ptr(self.normal),
-               L.ptr(q), nq, self.inv_h, self.h, int(k), float(stdv if stdv is not None else 0.0), L.ptr(idx), L.ptr(d2),
-               L.ptr(sdf), L.stream())
+        L.call("ngs_knn_tree_query", L.ptr(self.tree), self.tree.numel(), L.ptr(self.xyz), self.xyz.shape[0],
+               L.ptr(self.normal), L.ptr(q), nq, int(k), float(stdv if stdv is not None else 0.0), L.ptr(idx),
+               L.ptr(d2), L.ptr(sdf), L.stream())
         return idx, d2, sdf
 
 
