@@ -176,7 +176,8 @@ extern "C" int ngs_knn_sdf(ngs_grid g, const int64_t* start, const int32_t* sort
 // tenth of the scene off the surface reads ~10^5 empty cells and holds up its warp.  What bounds the tree
 // walk is the chain of box test -> choice of the nearest child -> next box test, 3 to 5 levels deep, and
 // the shuffles of the list.  Measured (60,000 points on a torus, 100,000 queries, 1 in 16 anywhere in the
-// cube around it, k = 8, signed distance): build and queries 0.65 ms, the grid walk 376 ms.
+// cube around it, k = 8, signed distance): build and queries 0.45 ms, the grid walk 376 ms (with
+// every point inserted one by one, and cells of 16 points instead of 2: 0.65 ms).
 //
 // Exactness: a box's squared distance is formed from lo - q or hi - q by the operations that form a
 // point's from p - q.  Each rounds monotonically, so no point of a box is nearer than its box, and skipping
@@ -217,10 +218,10 @@ extern "C" size_t ngs_knn_tree_bytes(int64_t n) {
   return (size_t)(knn_align(n * 16) + (t.off[t.levels - 1] + t.cnt[t.levels - 1]) * 32);
 }
 
-// Cells per axis 2^bits: about 16 points per occupied cell for points on a surface, at most 512.
+// Cells per axis 2^bits: about 2 points per occupied cell for points on a surface, at most 512.
 static int knn_tree_bits(int64_t n) {
   int b = 2;
-  while (b < 9 && ((int64_t)16 << (2 * b)) < n) b++;
+  while (b < 9 && ((int64_t)2 << (2 * b)) < n) b++;
   return b;
 }
 
@@ -364,6 +365,18 @@ NGS_DEV float knn_d2(float dx, float dy, float dz) {
   const float d = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
   return d == d ? d : INFINITY;
 }
+// Distance and index as one ordered number: the bits of a distance, which is never negative, order as the
+// distance does.
+NGS_DEV unsigned long long knn_key(float d, int i) {
+  return (unsigned long long)__float_as_uint(d) << 32 | (unsigned)i;
+}
+constexpr unsigned long long KNN_NONE = 0x7f8000007fffffffull;        // (infinity, INT_MAX): after every point
+
+// One step of a bitonic network over the warp: lane keeps the smaller of the pair (lane, lane ^ o) if `low`.
+NGS_DEV unsigned long long knn_exchange(unsigned long long v, int o, bool low) {
+  const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+  return (w < v) == low ? w : v;
+}
 // Distance along one axis from q to [lo, hi] (0 inside; a NaN query stays NaN).
 NGS_DEV float knn_gap(float lo, float hi, float q) { return q < lo ? lo - q : (q > hi ? q - hi : q - q); }
 
@@ -379,10 +392,9 @@ __global__ void __launch_bounds__(KNN_TREE_WARPS * 32) knn_tree_query_kernel(
   const int64_t warps = (int64_t)gridDim.x * KNN_TREE_WARPS;
   for (int64_t i = (int64_t)blockIdx.x * KNN_TREE_WARPS + w; i < nq; i += warps) {
     const float px = q[3 * i], py = q[3 * i + 1], pz = q[3 * i + 2];
-    float bd = INFINITY;                     // lane j: the j-th best, (infinity, INT_MAX) while there is none
-    int bi = 0x7fffffff;
-    float kd = INFINITY;                     // the k-th best
-    int ki = 0x7fffffff;
+    unsigned long long mine = KNN_NONE;      // lane j: the j-th best point
+    unsigned long long last = KNN_NONE;      // the k-th best
+    float kd = INFINITY;
     int lev = t.levels - 1, node = 0;        // node: the parent whose children at level lev are tested
     bool fresh = true;
     while (lev < t.levels) {
@@ -406,8 +418,7 @@ __global__ void __launch_bounds__(KNN_TREE_WARPS * 32) knn_tree_query_kernel(
       // the nearest child still to visit; one beyond the k-th best ends the node
       const float d = s_d[w][lev][lane];
       const unsigned left = s_left[w][lev];
-      const bool mine = (left >> lane) & 1u;
-      const unsigned key = mine ? __float_as_uint(d) : 0xffffffffu;
+      const unsigned key = (left >> lane) & 1u ? __float_as_uint(d) : 0xffffffffu;
       const unsigned best = __reduce_min_sync(0xffffffffu, key);
       if (left == 0u || __uint_as_float(best) > kd) {
         lev++;
@@ -424,38 +435,42 @@ __global__ void __launch_bounds__(KNN_TREE_WARPS * 32) knn_tree_query_kernel(
         fresh = true;
         continue;
       }
-      // a leaf: one point per lane, those that enter the list one after another
+      // a leaf: one point per lane.  A few that enter the list are inserted one after another; more (the
+      // first leaf, above all) are sorted and merged with the list, some 150 instructions against 25 each
       const int64_t c = (int64_t)child * 32 + lane;
-      float pd = INFINITY;
-      int pi = 0x7fffffff;
+      unsigned long long pt = KNN_NONE;
       if (c < t.n) {
         const float4 p = __ldg(t.pts + c);
-        pd = knn_d2(p.x - px, p.y - py, p.z - pz);
-        pi = __float_as_int(p.w);
+        pt = knn_key(knn_d2(p.x - px, p.y - py, p.z - pz), __float_as_int(p.w));
       }
-      unsigned cand = __ballot_sync(0xffffffffu, pi != 0x7fffffff && knn_less(pd, pi, kd, ki));
+      unsigned cand = __ballot_sync(0xffffffffu, pt < last);
+      if (__popc(cand) > 6) {
+#pragma unroll
+        for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+          for (int o = size >> 1; o > 0; o >>= 1) pt = knn_exchange(pt, o, ((lane & o) == 0) == ((lane & size) == 0));
+        // the list and the reversed leaf: the 32 smallest of both form a bitonic sequence
+        pt = __shfl_xor_sync(0xffffffffu, pt, 31);
+        mine = pt < mine ? pt : mine;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mine = knn_exchange(mine, o, (lane & o) == 0);
+        last = __shfl_sync(0xffffffffu, mine, k - 1);
+        cand = 0u;
+      }
       while (cand) {
-        const int from = __ffs(cand) - 1;
-        const float nd = __shfl_sync(0xffffffffu, pd, from);
-        const int ni = __shfl_sync(0xffffffffu, pi, from);
-        const unsigned before = __ballot_sync(0xffffffffu, knn_less(bd, bi, nd, ni));
-        const float ud = __shfl_up_sync(0xffffffffu, bd, 1);
-        const int ui = __shfl_up_sync(0xffffffffu, bi, 1);
-        const int at = __popc(before);       // the list is sorted: the lanes before are 0 .. at - 1
-        if (lane > at) {
-          bd = ud;
-          bi = ui;
-        } else if (lane == at) {
-          bd = nd;
-          bi = ni;
-        }
-        kd = __shfl_sync(0xffffffffu, bd, k - 1);
-        ki = __shfl_sync(0xffffffffu, bi, k - 1);
+        const unsigned long long p = __shfl_sync(0xffffffffu, pt, __ffs(cand) - 1);
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, mine, 1);
+        const int at = __popc(__ballot_sync(0xffffffffu, mine < p));     // sorted: lanes 0 .. at - 1
+        mine = lane > at ? up : (lane == at ? p : mine);
+        last = __shfl_sync(0xffffffffu, mine, k - 1);
         cand &= cand - 1u;
-        cand &= __ballot_sync(0xffffffffu, knn_less(pd, pi, kd, ki));
+        cand &= __ballot_sync(0xffffffffu, pt < last);
       }
+      kd = __uint_as_float((unsigned)(last >> 32));
     }
-    const bool have = lane < k && bi != 0x7fffffff;
+    const float bd = __uint_as_float((unsigned)(mine >> 32));
+    const int bi = (int)(unsigned)mine;
+    const bool have = lane < k && mine != KNN_NONE;
     if (lane < k) {
       if (idx_out) idx_out[i * k + lane] = have ? bi : -1;
       if (d2_out) d2_out[i * k + lane] = have && px + py + pz != px + py + pz && bd == INFINITY ? NAN : bd;
