@@ -19,6 +19,7 @@
 // fence) and "empty" (tcgen05.commit of the MMAs that read the stage).  Every wait is bounded; on timeout the kernel records NGS_ERR_TIMEOUT,
 // stops issuing, waits (bounded) for its MMAs and releases its TMEM before returning.
 #include <cstdint>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "ngs_common.cuh"
@@ -506,7 +507,7 @@ __global__ void conv_wgrad_reduce_kernel(const float* __restrict__ part, int K, 
 // ----------------------------------------------------------------------------- CUDA-core path
 // FP32 inputs (the reference's path outside autocast is an FP32 cuBLAS GEMM, so FP32 stays FP32 here)
 // and 16-bit shapes the tensor-core tiles do not take (kdim not a multiple of 8, ncols not a multiple
-// of 16): one thread per output element, FP32 accumulation.
+// of 16): FP32 multiply-adds on 4 x 4 outputs per thread, both operands staged through shared memory.
 template <typename T>
 NGS_DEV float to_f(T v) { return (float)v; }
 template <>
@@ -521,41 +522,246 @@ NGS_DEV void put(void* out, int64_t i, float v, bool f32) {
   else static_cast<float*>(out)[i] = v;
 }
 
+// Elements c .. c + 3 of a row of len elements as FP32, zero past its end; one 16-byte load for FP32
+// rows that allow it (vec: len a multiple of 4 and the base 16-byte aligned).
 template <typename T>
-__global__ void conv_gather_gemm_simt_kernel(const T* __restrict__ x, int64_t n_src, int kdim,
-                                             const int32_t* __restrict__ table, int64_t n_rows, int K,
-                                             const T* __restrict__ bt, int ncols, void* out, int out_f32) {
-  const int64_t total = n_rows * ncols;
-  for (int64_t e = ngs_gtid(); e < total; e += ngs_gstride()) {
-    const int64_t r = e / ncols;
-    const int n = (int)(e % ncols);
-    float acc = 0.f;
-    for (int k = 0; k < K; k++) {
-      const int32_t src = table[r * K + k];
-      if (src < 0 || src >= n_src) continue;
-      const T* xr = x + (int64_t)src * kdim;
-      const T* br = bt + ((int64_t)k * ncols + n) * kdim;
-      for (int c = 0; c < kdim; c++) acc += to_f(xr[c]) * to_f(br[c]);
+NGS_DEV float4 load4(const T* __restrict__ row, int c, int len, bool vec) {
+  if constexpr (sizeof(T) == 4) {
+    if (vec) return c < len ? __ldg(reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float4 v;
+  v.x = c < len ? to_f(row[c]) : 0.f;
+  v.y = c + 1 < len ? to_f(row[c + 1]) : 0.f;
+  v.z = c + 2 < len ? to_f(row[c + 2]) : 0.f;
+  v.w = c + 3 < len ? to_f(row[c + 3]) : 0.f;
+  return v;
+}
+NGS_DEV bool finite4(float4 v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w); }
+
+// A tile of BM output rows x BN columns.  Per kernel offset that some row of the tile has, and per slice
+// of CK channels: the rows gathered and the offset's weights into shared memory (both with the channel
+// outermost), the next stage's loads in flight in registers while this one is multiplied.  A thread's
+// sums run over the offsets and channels in order, as one thread per output would run them.  A missing
+// row is staged as zeros, which adds nothing unless a weight is infinite or NaN: a stage with such a
+// weight takes the rows one by one.
+// What bounds it is the gather's latency over some 30 stages a tile.  Measured, FP32, 16 -> 32 channels,
+// 44,595 rows, 702,000 pairs: forward 0.063 ms and input gradient 0.105 ms, against 0.83 ms each with one
+// thread per output that reads its rows and weights for itself.
+template <typename T, int BM, int BN, int CK>
+__global__ void __launch_bounds__(BM* BN / 16) conv_gather_gemm_simt_kernel(
+    const T* __restrict__ x, int64_t n_src, int kdim, const int32_t* __restrict__ table, int64_t n_rows, int K,
+    const T* __restrict__ bt, int ncols, void* out, int out_f32, int vec) {
+  constexpr int NT = BM * BN / 16;
+  constexpr int NA = BM * CK / 4 / NT, NB = (BN * CK / 4 + NT - 1) / NT;
+  __shared__ __align__(16) float As[CK][BM + 4];
+  __shared__ __align__(16) float Bs[CK][BN + 4];
+  __shared__ int s_valid[BM];
+  __shared__ unsigned s_any[(conv::KMAX + 31) / 32];
+  const int t = threadIdx.x, tx = t % (BN / 4), ty = t / (BN / 4);
+  const int64_t r0 = (int64_t)blockIdx.x * BM;
+  const int n0 = blockIdx.y * BN;
+  for (int k = t; k < (conv::KMAX + 31) / 32; k += NT) s_any[k] = 0u;
+  __syncthreads();
+  const int rows = (int)min((int64_t)BM, n_rows - r0);
+  for (int e = t; e < rows * K; e += NT) {
+    const int32_t src = table[r0 * K + e];
+    const int k = e % K;
+    if (src >= 0 && src < n_src) atomicOr(&s_any[k >> 5], 1u << (k & 31));
+  }
+  __syncthreads();
+  auto next_k = [&](int k) {
+    for (k++; k < K; k++)
+      if ((s_any[k >> 5] >> (k & 31)) & 1u) break;
+    return k;
+  };
+  float4 ra[NA], rb[NB];
+  bool va = false;
+  auto fetch = [&](int k, int c0) {
+#pragma unroll
+    for (int j = 0; j < NA; j++) {
+      const int e = t + j * NT, row = e % BM, c = c0 + e / BM * 4;
+      const int32_t src = row < rows ? __ldg(table + (r0 + row) * K + k) : -1;
+      const bool ok = src >= 0 && src < n_src;
+      if (j == 0) va = ok;                            // thread t < BM stages row t first
+      ra[j] = ok ? load4<T>(x + (int64_t)src * kdim, c, kdim, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    put<T>(out, e, acc, out_f32 != 0);
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+      const int e = t + j * NT, n = e % BN, c = c0 + e / BN * 4;
+      rb[j] = e < BN * CK / 4 && n0 + n < ncols ? load4<T>(bt + ((int64_t)k * ncols + n0 + n) * kdim, c, kdim, vec)
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+  int k = next_k(-1), c0 = 0;
+  if (k < K) fetch(k, c0);
+  while (k < K) {
+    int odd = 0;
+#pragma unroll
+    for (int j = 0; j < NA; j++) {
+      const int e = t + j * NT, row = e % BM, c = e / BM * 4;
+      As[c][row] = ra[j].x;
+      As[c + 1][row] = ra[j].y;
+      As[c + 2][row] = ra[j].z;
+      As[c + 3][row] = ra[j].w;
+    }
+    if (t < BM) s_valid[t] = va;
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+      const int e = t + j * NT, n = e % BN, c = e / BN * 4;
+      if (e < BN * CK / 4) {
+        Bs[c][n] = rb[j].x;
+        Bs[c + 1][n] = rb[j].y;
+        Bs[c + 2][n] = rb[j].z;
+        Bs[c + 3][n] = rb[j].w;
+        odd |= !finite4(rb[j]);
+      }
+    }
+    odd = __syncthreads_or(odd);
+    c0 += CK;
+    if (c0 >= kdim) {
+      c0 = 0;
+      k = next_k(k);
+    }
+    if (k < K) fetch(k, c0);                          // the next stage, while this one is multiplied
+    bool use[4] = {true, true, true, true};
+    if (odd) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) use[i] = s_valid[ty * 4 + i] != 0;
+    }
+#pragma unroll 16
+    for (int c = 0; c < CK; c++) {
+      const float4 a4 = *reinterpret_cast<const float4*>(&As[c][ty * 4]);
+      const float4 b4 = *reinterpret_cast<const float4*>(&Bs[c][tx * 4]);
+      const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
+      if (!odd) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (use[i]) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int row = ty * 4 + i;
+    if (row >= rows) continue;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int n = n0 + tx * 4 + j;
+      if (n < ncols) put<T>(out, (r0 + row) * ncols + n, acc[i][j], out_f32 != 0);
+    }
   }
 }
 
-template <typename T>
-__global__ void conv_wgrad_simt_kernel(const T* __restrict__ x, const T* __restrict__ gy, int64_t n_in, int64_t n_out,
-                                       int cin, int cout, const int32_t* __restrict__ nbmaps,
-                                       const int64_t* __restrict__ starts, int in_col, int K, void* out, int out_f32) {
-  const int64_t total = (int64_t)K * cin * cout;
-  for (int64_t e = ngs_gtid(); e < total; e += ngs_gstride()) {
-    const int k = (int)(e / ((int64_t)cin * cout));
-    const int ci = (int)((e / cout) % cin), co = (int)(e % cout);
-    float acc = 0.f;
-    for (int64_t p = starts[k]; p < starts[k + 1]; p++) {
-      const int32_t i = nbmaps[2 * p + in_col], o = nbmaps[2 * p + 1 - in_col];
-      if (i < 0 || i >= n_in || o < 0 || o >= n_out) continue;
-      acc += to_f(x[(int64_t)i * cin + ci]) * to_f(gy[(int64_t)o * cout + co]);
+// Weight gradient: per offset a BM x BN tile of channels, the offset's pairs split over blockIdx.x (a
+// partial per split, added in split order by conv_wgrad_reduce_kernel), a stage of 64 pairs in shared
+// memory.  Tiles smaller than 128 threads' work are kept by several groups of threads, each on its share
+// of a stage's pairs, added in group order.  A pair outside the feature maps is staged as two rows of
+// zeros.  Measured on the same layer: 0.05 ms, against 7.8 ms with one thread per weight walking all pairs
+// of its offset; the partial sums are short, so the error against 64 bits fell from 2.9e-6 to 4.1e-7.
+constexpr int SIMT_PAIRS = 64;
+
+template <typename T, int BM, int BN>
+__global__ void __launch_bounds__(BM* BN / 16 < 128 ? 128 : BM * BN / 16) conv_wgrad_simt_kernel(
+    const T* __restrict__ x, const T* __restrict__ gy, int64_t n_in, int64_t n_out, int cin, int cout,
+    const int32_t* __restrict__ nbmaps, const int64_t* __restrict__ starts, int in_col, float* __restrict__ part,
+    void* out, int out_f32, int vec_x, int vec_y) {
+  constexpr int TT = BM * BN / 16, NT = TT < 128 ? 128 : TT, GROUPS = NT / TT;
+  constexpr int NA = SIMT_PAIRS * BM / 4 / NT, NB = SIMT_PAIRS * BN / 4 / NT;
+  union Stage {
+    struct {
+      float a[SIMT_PAIRS][BM];
+      float b[SIMT_PAIRS][BN];
+    } s;
+    float sum[GROUPS][BM * BN];
+  };
+  __shared__ __align__(16) Stage sh;
+  const int t = threadIdx.x, g = t / TT, tx = t % TT % (BN / 4), ty = t % TT / (BN / 4);
+  const int k = blockIdx.y, split = blockIdx.x, splits = gridDim.x;
+  const int nt = (cout + BN - 1) / BN, m0 = blockIdx.z / nt * BM, n0 = blockIdx.z % nt * BN;
+  const int64_t first = starts[k], count = starts[k + 1] - first;
+  const int64_t chunks = (count + SIMT_PAIRS - 1) / SIMT_PAIRS;
+  const int64_t p_end = first + min(count, chunks * (split + 1) / splits * SIMT_PAIRS);
+  int64_t p0 = first + chunks * split / splits * SIMT_PAIRS;
+  float4 ra[NA], rb[NB];
+  auto fetch = [&](int64_t p) {
+#pragma unroll
+    for (int j = 0; j < NA; j++) {
+      const int e = t + j * NT, c = e % (BM / 4) * 4;
+      const int64_t q = p + e / (BM / 4);
+      ra[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (q < p_end) {
+        const int32_t i = nbmaps[2 * q + in_col], o = nbmaps[2 * q + 1 - in_col];
+        if (i >= 0 && i < n_in && o >= 0 && o < n_out) ra[j] = load4<T>(x + (int64_t)i * cin, m0 + c, cin, vec_x);
+      }
     }
-    put<T>(out, e, acc, out_f32 != 0);
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+      const int e = t + j * NT, c = e % (BN / 4) * 4;
+      const int64_t q = p + e / (BN / 4);
+      rb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (q < p_end) {
+        const int32_t i = nbmaps[2 * q + in_col], o = nbmaps[2 * q + 1 - in_col];
+        if (i >= 0 && i < n_in && o >= 0 && o < n_out) rb[j] = load4<T>(gy + (int64_t)o * cout, n0 + c, cout, vec_y);
+      }
+    }
+  };
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+  if (p0 < p_end) fetch(p0);
+  for (; p0 < p_end; p0 += SIMT_PAIRS) {
+#pragma unroll
+    for (int j = 0; j < NA; j++) {
+      const int e = t + j * NT;
+      *reinterpret_cast<float4*>(&sh.s.a[e / (BM / 4)][e % (BM / 4) * 4]) = ra[j];
+    }
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+      const int e = t + j * NT;
+      *reinterpret_cast<float4*>(&sh.s.b[e / (BN / 4)][e % (BN / 4) * 4]) = rb[j];
+    }
+    __syncthreads();
+    if (p0 + SIMT_PAIRS < p_end) fetch(p0 + SIMT_PAIRS);
+#pragma unroll 8
+    for (int p = g; p < SIMT_PAIRS; p += GROUPS) {
+      const float4 a4 = *reinterpret_cast<const float4*>(&sh.s.a[p][ty * 4]);
+      const float4 b4 = *reinterpret_cast<const float4*>(&sh.s.b[p][tx * 4]);
+      const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) sh.sum[g][(ty * 4 + i) * BN + tx * 4 + j] = acc[i][j];
+  __syncthreads();
+  for (int e = t; e < BM * BN; e += NT) {
+    const int m = m0 + e / BN, n = n0 + e % BN;
+    if (m >= cin || n >= cout) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int h = 0; h < GROUPS; h++) v += sh.sum[h][e];
+    if (part) part[(((int64_t)k * splits + split) * cin + m) * cout + n] = v;
+    else put<T>(out, ((int64_t)k * cin + m) * cout + n, v, out_f32 != 0);
   }
 }
 
@@ -583,13 +789,77 @@ void tile_plan(int n, int& stages, uint32_t& stage_bytes, size_t& smem) {
   smem = (size_t)stages * stage_bytes + 1024;        // + alignment of the first stage to 1024 bytes
 }
 
+// Column tile of the CUDA-core kernels: the smallest of 16, 32 and 64 that holds the columns (a narrower
+// tile than the columns need would gather the rows once more, a wider one multiplies zeros).
+template <typename T, int BM, int BN>
+int simt_gemm_tile(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K, const void* bt,
+                   int ncols, void* out, int out_f32, cudaStream_t st) {
+  const dim3 grid((unsigned)((n_rows + BM - 1) / BM), (unsigned)((ncols + BN - 1) / BN));
+  ngs_count_launch();
+  // slices of 32 channels where there are more than 16: half the stages, and a stage is a round trip
+  const int vec = kdim % 4 == 0 && aligned16(x) && aligned16(bt);
+  if (kdim <= 16)
+    conv_gather_gemm_simt_kernel<T, BM, BN, 16><<<grid, BM * BN / 16, 0, st>>>(
+        static_cast<const T*>(x), n_src, kdim, table, n_rows, K, static_cast<const T*>(bt), ncols, out, out_f32, vec);
+  else
+    conv_gather_gemm_simt_kernel<T, BM, BN, 32><<<grid, BM * BN / 16, 0, st>>>(
+        static_cast<const T*>(x), n_src, kdim, table, n_rows, K, static_cast<const T*>(bt), ncols, out, out_f32, vec);
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}
+
 template <typename T>
 int simt_gemm(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K, const void* bt,
               int ncols, void* out, int out_f32, cudaStream_t st) {
+  if (ncols <= 16) return simt_gemm_tile<T, 64, 16>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
+  if (ncols <= 32) return simt_gemm_tile<T, 64, 32>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
+  return simt_gemm_tile<T, 64, 64>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
+}
+
+// Splits of the pairs: at least 512 pairs each (CUDA cores) or 2,048 (tensor cores), at most 64.
+int wgrad_splits(int64_t max_pairs, int64_t least) {
+  const int64_t s = (max_pairs + least - 1) / least;
+  return (int)(s < 1 ? 1 : (s > 64 ? 64 : s));
+}
+
+template <typename T, int BM, int BN>
+void simt_wgrad_tile(const void* x, const void* gy, int64_t n_in, int64_t n_out, int cin, int cout,
+                     const int32_t* nbmaps, const int64_t* starts, int in_col, int K, int splits, float* part,
+                     void* out, int out_f32, cudaStream_t st) {
+  const dim3 grid((unsigned)splits, (unsigned)K, (unsigned)(((cin + BM - 1) / BM) * ((cout + BN - 1) / BN)));
   ngs_count_launch();
-  conv_gather_gemm_simt_kernel<T><<<ngs_blocks(n_rows * ncols, 256), 256, 0, st>>>(
-      static_cast<const T*>(x), n_src, kdim, table, n_rows, K, static_cast<const T*>(bt), ncols, out, out_f32);
+  conv_wgrad_simt_kernel<T, BM, BN><<<grid, BM * BN / 16 < 128 ? 128 : BM * BN / 16, 0, st>>>(
+      static_cast<const T*>(x), static_cast<const T*>(gy), n_in, n_out, cin, cout, nbmaps, starts, in_col, part, out,
+      out_f32, cin % 4 == 0 && aligned16(x), cout % 4 == 0 && aligned16(gy));
+}
+
+template <typename T>
+int simt_wgrad(const void* x, const void* gy, int64_t n_in, int64_t n_out, int cin, int cout, const int32_t* nbmaps,
+               const int64_t* starts, int in_col, int K, int64_t max_pairs, void* out, int out_f32, void* ws,
+               size_t ws_bytes, cudaStream_t st) {
+  // without a workspace for the partials, one split per offset
+  int splits = wgrad_splits(max_pairs, 512);
+  if (!ws || ws_bytes < (size_t)K * splits * cin * cout * sizeof(float) || !aligned16(ws)) splits = 1;
+  float* part = splits > 1 ? static_cast<float*>(ws) : nullptr;
+  auto go = [&](auto bm, auto bn) {
+    simt_wgrad_tile<T, decltype(bm)::value, decltype(bn)::value>(x, gy, n_in, n_out, cin, cout, nbmaps, starts, in_col,
+                                                                 K, splits, part, out, out_f32, st);
+  };
+  auto with_bm = [&](auto bm) {
+    if (cout <= 16) go(bm, std::integral_constant<int, 16>{});
+    else if (cout <= 32) go(bm, std::integral_constant<int, 32>{});
+    else go(bm, std::integral_constant<int, 64>{});
+  };
+  if (cin <= 16) with_bm(std::integral_constant<int, 16>{});
+  else if (cin <= 32) with_bm(std::integral_constant<int, 32>{});
+  else with_bm(std::integral_constant<int, 64>{});
   NGS_CHECK_LAUNCH();
+  if (part) {
+    ngs_count_launch();
+    conv_wgrad_reduce_kernel<<<ngs_blocks((int64_t)K * cin * cout, 256), 256, 0, st>>>(
+        part, K, splits, (int64_t)cin * cout, out, out_f32, std::is_same<T, __nv_bfloat16>::value);
+    NGS_CHECK_LAUNCH();
+  }
   return NGS_OK;
 }
 
@@ -653,10 +923,7 @@ extern "C" int ngs_conv_gather_gemm(const void* x, int64_t n_src, int kdim, cons
 }
 
 extern "C" size_t ngs_conv_weight_grad_ws_bytes(int K, int cin, int cout, int64_t max_pairs) {
-  int64_t splits = (max_pairs + 2047) / 2048;
-  if (splits < 1) splits = 1;
-  if (splits > 64) splits = 64;
-  return (size_t)K * splits * cin * cout * sizeof(float);
+  return (size_t)K * wgrad_splits(max_pairs, 512) * cin * cout * sizeof(float);
 }
 
 extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const void* gy, int64_t n_out, int cout,
@@ -668,26 +935,19 @@ extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const 
       (max_pairs > 0 && !nbmaps) || (n_in > 0 && !x) || (n_out > 0 && !gy))
     return NGS_ERR_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)s;
-  const int64_t total = (int64_t)K * cin * cout;
   const bool tc = (dtype == NGS_F16 || dtype == NGS_BF16) && cout % 16 == 0 && aligned16(grad_w);
   if (!tc) {
-    ngs_count_launch();
     if (dtype == NGS_F32)
-      conv_wgrad_simt_kernel<float><<<ngs_blocks(total, 256), 256, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(gy), n_in, n_out, cin, cout, nbmaps, starts_dev,
-          in_col, K, grad_w, 1);
-    else if (dtype == NGS_BF16)
-      conv_wgrad_simt_kernel<__nv_bfloat16><<<ngs_blocks(total, 256), 256, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gy), n_in, n_out, cin, cout, nbmaps,
-          starts_dev, in_col, K, grad_w, out_f32);
-    else
-      conv_wgrad_simt_kernel<__half><<<ngs_blocks(total, 256), 256, 0, st>>>(
-          static_cast<const __half*>(x), static_cast<const __half*>(gy), n_in, n_out, cin, cout, nbmaps, starts_dev,
-          in_col, K, grad_w, out_f32);
-    NGS_CHECK_LAUNCH();
-    return NGS_OK;
+      return simt_wgrad<float>(x, gy, n_in, n_out, cin, cout, nbmaps, starts_dev, in_col, K, max_pairs, grad_w, 1, ws,
+                               ws_bytes, st);
+    if (dtype == NGS_BF16)
+      return simt_wgrad<__nv_bfloat16>(x, gy, n_in, n_out, cin, cout, nbmaps, starts_dev, in_col, K, max_pairs, grad_w,
+                                       out_f32, ws, ws_bytes, st);
+    return simt_wgrad<__half>(x, gy, n_in, n_out, cin, cout, nbmaps, starts_dev, in_col, K, max_pairs, grad_w, out_f32,
+                              ws, ws_bytes, st);
   }
-  const size_t need = ngs_conv_weight_grad_ws_bytes(K, cin, cout, max_pairs);
+  const int splits = wgrad_splits(max_pairs, 2048);
+  const size_t need = (size_t)K * splits * cin * cout * sizeof(float);
   if (!ws || ws_bytes < need) return NGS_ERR_OOM;
   WeightGrad g{};
   g.x = static_cast<const uint16_t*>(x);
@@ -700,7 +960,7 @@ extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const 
   g.starts = starts_dev;
   g.in_col = in_col;
   g.K = K;
-  g.splits = (int)(need / ((size_t)K * cin * cout * sizeof(float)));
+  g.splits = splits;
   g.m_tiles = (cin + conv::BM - 1) / conv::BM;
   g.part = static_cast<float*>(ws);
   g.mn = cin % 64 == 0 && cout % 64 == 0 && aligned16(x) && aligned16(gy);
@@ -715,7 +975,7 @@ extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const 
   conv_wgrad_kernel<<<grid, conv::THREADS, smem, st>>>(g);
   NGS_CHECK_LAUNCH();
   ngs_count_launch();
-  conv_wgrad_reduce_kernel<<<ngs_blocks(total, 256), 256, 0, st>>>(g.part, K, g.splits, (int64_t)cin * cout, grad_w,
+  conv_wgrad_reduce_kernel<<<ngs_blocks((int64_t)K * cin * cout, 256), 256, 0, st>>>(g.part, K, g.splits, (int64_t)cin * cout, grad_w,
                                                                   out_f32, g.bf16);
   NGS_CHECK_LAUNCH();
   return NGS_OK;
