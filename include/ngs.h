@@ -448,7 +448,9 @@ int ngs_mf_gram(const int64_t* t_ptr, const int32_t* t_point, const float* t_phi
  *   the device), -1 for none; key_col is the column of nbmaps that indexes the table; mid >= 0 sets
  *   table[row, mid] = row (the reference's forward takes the centre offset as the identity when the
  *   input and output sets are the same).
- * ngs_conv_gather_gemm: out[r, n] = sum_k sum_c x[table[r, k], c] * bt[k, n, c] (bt = the weights of
+ * ngs_conv_table_kmajor: the same entries with the offset outermost, int32 [K, n_rows] (written and read in
+ *   order: the layout to use unless a table already exists).
+ * ngs_conv_gather_gemm (tables [n_rows, K]), ngs_conv_gather_gemm_kmajor ([K, n_rows]): out[r, n] = sum_k sum_c x[table[r, k], c] * bt[k, n, c] (bt = the weights of
  *   every offset with the reduction index innermost), one kernel, every output row written once
  *   (FP32 out when out_f32, else the input type).  Forward: x = input, bt = W^T per offset
  *   (ngs_conv_transpose_weight); input gradient: x = output gradient, table of the other column,
@@ -460,10 +462,15 @@ int ngs_mf_gram(const int64_t* t_ptr, const int32_t* t_point, const float* t_phi
 enum { NGS_F16 = 0, NGS_BF16 = 1, NGS_F32 = 2 };
 int ngs_conv_table(const int32_t* nbmaps, const int64_t* starts_dev, int K, int key_col, int64_t n_rows, int mid,
                    int32_t* table, ngs_stream s);
+int ngs_conv_table_kmajor(const int32_t* nbmaps, const int64_t* starts_dev, int K, int key_col, int64_t n_rows, int mid,
+                          int32_t* table, ngs_stream s);
 int ngs_conv_transpose_weight(const void* w, int K, int a, int b, int dtype, void* wt, ngs_stream s);
 int ngs_conv_tensor_core_ok(int kdim, int ncols, int dtype);
 int ngs_conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K,
                          const void* bt, int ncols, int dtype, void* out, int out_f32, int* error_dev, ngs_stream s);
+int ngs_conv_gather_gemm_kmajor(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K,
+                                const void* bt, int ncols, int dtype, void* out, int out_f32, int* error_dev,
+                                ngs_stream s);
 size_t ngs_conv_weight_grad_ws_bytes(int K, int cin, int cout, int64_t max_pairs);
 int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const void* gy, int64_t n_out, int cout,
                          const int32_t* nbmaps, const int64_t* starts_dev, int K, int64_t max_pairs, int in_col,

@@ -32,15 +32,9 @@ constexpr int UK = 16;               // UMMA K of kind::f16
 constexpr int PRODUCERS = 256;       // warps 0-7
 constexpr int THREADS = PRODUCERS + 32;
 constexpr int KMAX = 128;            // kernel offsets (5^3 = 125 at most)
-constexpr unsigned long long WAIT_NS = 2000000000ull;   // bound of one mbarrier wait (2 s)
+constexpr long long WAIT_CYCLES = 4000000000ll;         // bound of one mbarrier wait (2 s or more)
 
 NGS_DEV uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-NGS_DEV unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 
 NGS_DEV void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -61,10 +55,10 @@ NGS_DEV bool mbar_try(uint64_t* bar, uint32_t parity) {
 // thread of the CTA already gave up (abort flag in shared memory).
 NGS_DEV bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
   if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = now_ns();
+  const long long t0 = clock64();
   while (!mbar_try(bar, parity)) {
     if (*abort) return false;
-    if (now_ns() - t0 > WAIT_NS) {
+    if (clock64() - t0 > WAIT_CYCLES) {
       *abort = 1;
       return false;
     }
@@ -117,6 +111,19 @@ NGS_DEV void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;"
 // Generic-proxy stores to shared memory become visible to the tensor core (async proxy).
 NGS_DEV void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// 16 bytes from global to shared memory without passing through registers; zeros when !have.
+NGS_DEV void cp_async16(uint32_t dst, const void* src, bool have) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %2, 0;\n\tcp.async.cg.shared.global [%0], [%1], 16, p;\n\t}" ::"r"(dst),
+      "l"(src), "r"((uint32_t)have)
+      : "memory");
+}
+NGS_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+NGS_DEV void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
 // TMEM allocation by one whole warp; the column base lands in *dst (shared memory).
 NGS_DEV void tmem_alloc(uint32_t* dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(ncols)
@@ -145,41 +152,53 @@ NGS_DEV uint32_t sw128(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)
 }  // namespace conv
 
 // ----------------------------------------------------------------------------- gather tables
-// table[row, k] = the source row paired with `row` at offset k (-1: none).  Pairs of offset k are
-// nbmaps[starts[k] .. starts[k+1]) as (c0, c1) int32 pairs; key_col picks the column that indexes the
-// table rows, the other column is the source.  mid >= 0: table[row, mid] = row for every row (the
-// reference's forward computes that offset as one dense product over all rows).
+// Entry (row, k) of a table, at row * row_stride + k * k_stride: the source row paired with `row` at
+// offset k (-1: none).  Pairs of offset k are nbmaps[starts[k] .. starts[k+1]) as (c0, c1) int32 pairs;
+// key_col picks the column that indexes the table rows, the other column is the source.  mid >= 0:
+// entry (row, mid) = row for every row (the reference's forward computes that offset as one dense
+// product over all rows).
+// The pairs of an offset usually come in the order of their rows, so with the offset outermost (k_stride
+// = n_rows) a warp's entries are neighbours in memory, and so are a tile's when they are read; with the row
+// outermost every entry is a 32-byte sector of its own.  1.3M rows, 24M pairs: 0.087 ms against 0.52.
 __global__ void conv_table_kernel(const int32_t* __restrict__ nbmaps, const int64_t* __restrict__ starts, int K,
-                                  int key_col, int64_t n_rows, int mid, int32_t* __restrict__ table) {
-  const int64_t total = starts[K];
-  for (int64_t p = ngs_gtid(); p < total; p += ngs_gstride()) {
-    int lo = 0, hi = K - 1;                    // offset of pair p: last k with starts[k] <= p
-    while (lo < hi) {
-      const int m = (lo + hi + 1) >> 1;
-      if (starts[m] <= p) lo = m; else hi = m - 1;
-    }
-    if (lo == mid) continue;
+                                  int key_col, int64_t n_rows, int64_t row_stride, int64_t k_stride, int mid,
+                                  int32_t* __restrict__ table) {
+  const int k = blockIdx.y;
+  const int64_t first = starts[k], end = starts[k + 1];
+  if (k == mid) {
+    for (int64_t r = ngs_gtid(); r < n_rows; r += ngs_gstride()) table[r * row_stride + k * k_stride] = (int32_t)r;
+    return;
+  }
+  for (int64_t p = first + ngs_gtid(); p < end; p += ngs_gstride()) {
     const int32_t key = nbmaps[2 * p + key_col], src = nbmaps[2 * p + 1 - key_col];
     if (key < 0 || key >= n_rows) continue;    // the reference's scatter skips negative targets
-    table[(int64_t)key * K + lo] = src < 0 ? -1 : src;
+    table[key * row_stride + k * k_stride] = src < 0 ? -1 : src;
   }
-  if (mid >= 0)
-    for (int64_t r = ngs_gtid(); r < n_rows; r += ngs_gstride()) table[r * K + mid] = (int32_t)r;
+}
+
+static int conv_table(const int32_t* nbmaps, const int64_t* starts_dev, int K, int key_col, int64_t n_rows,
+                      int64_t row_stride, int64_t k_stride, int mid, int32_t* table, cudaStream_t st) {
+  if (K < 1 || K > 128 || (key_col != 0 && key_col != 1) || n_rows < 0 || mid >= K || !starts_dev ||
+      (n_rows > 0 && !table))
+    return NGS_ERR_INVALID_ARG;
+  if (n_rows > 0 && cudaMemsetAsync(table, 0xFF, (size_t)n_rows * K * sizeof(int32_t), st) != cudaSuccess)
+    return ngs_set_cuda_error(cudaGetLastError());
+  // the pair counts are on the device: about one thread per row and offset
+  const dim3 grid(ngs_blocks(n_rows > 0 ? n_rows : 1, 256, 8), (unsigned)K);
+  ngs_count_launch();
+  conv_table_kernel<<<grid, 256, 0, st>>>(nbmaps, starts_dev, K, key_col, n_rows, row_stride, k_stride, mid, table);
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
 }
 
 extern "C" int ngs_conv_table(const int32_t* nbmaps, const int64_t* starts_dev, int K, int key_col, int64_t n_rows,
                               int mid, int32_t* table, ngs_stream s) {
-  if (K < 1 || K > 128 || (key_col != 0 && key_col != 1) || n_rows < 0 || mid >= K || !starts_dev ||
-      (n_rows > 0 && !table))
-    return NGS_ERR_INVALID_ARG;
-  cudaStream_t st = (cudaStream_t)s;
-  if (n_rows > 0 && cudaMemsetAsync(table, 0xFF, (size_t)n_rows * K * sizeof(int32_t), st) != cudaSuccess)
-    return ngs_set_cuda_error(cudaGetLastError());
-  ngs_count_launch();
-  conv_table_kernel<<<ngs_blocks(n_rows > 0 ? n_rows * 4 : 1, 256, 16), 256, 0, st>>>(nbmaps, starts_dev, K, key_col,
-                                                                                      n_rows, mid, table);
-  NGS_CHECK_LAUNCH();
-  return NGS_OK;
+  return conv_table(nbmaps, starts_dev, K, key_col, n_rows, K, 1, mid, table, (cudaStream_t)s);
+}
+
+extern "C" int ngs_conv_table_kmajor(const int32_t* nbmaps, const int64_t* starts_dev, int K, int key_col,
+                                     int64_t n_rows, int mid, int32_t* table, ngs_stream s) {
+  return conv_table(nbmaps, starts_dev, K, key_col, n_rows, 1, n_rows, mid, table, (cudaStream_t)s);
 }
 
 // ----------------------------------------------------------------------------- the tile kernel
@@ -187,7 +206,9 @@ extern "C" int ngs_conv_table(const int32_t* nbmaps, const int64_t* starts_dev, 
 // every A_s (128 x 64) and B_s (N x 64) filled by the producers straight into a shared-memory stage
 // (K-major, 128-byte swizzle), accumulated in TMEM by tcgen05.mma, and handed to the epilogue.
 // Fill: the source of the tiles -- fill(step, a, b, tid) stores the stage's A and B rows (zeros where
-// there is no data) and returns the number of valid reduction elements of the step (<= 64).
+// there is no data) and returns the number of valid reduction elements of the step (<= 64).  ASYNC: fill
+// only issues asynchronous copies; the stage is handed over AHEAD steps later, so that a producer has the
+// copies of AHEAD + 1 stages in flight (the ring has at least AHEAD + 1 stages).
 // Store: store(row, col, v[16]) takes 16 consecutive accumulator columns of one tile row.
 namespace conv {
 
@@ -199,8 +220,9 @@ struct TileShape {
 };
 
 constexpr uint32_t A_BYTES = BM * 128;   // 16 KB
+constexpr int AHEAD = 2;
 
-template <typename Fill, typename Store>
+template <bool ASYNC, typename Fill, typename Store>
 NGS_DEV void run_tile(const TileShape& t, uint8_t* smem, Fill& fill, Store& store, int bf16, int* error,
                       bool mn_major = false) {
   __shared__ uint64_t full_bar[8], empty_bar[8], done_bar;
@@ -212,7 +234,7 @@ NGS_DEV void run_tile(const TileShape& t, uint8_t* smem, Fill& fill, Store& stor
   const uint32_t ncols_alloc = t.n <= 32 ? 32u : t.n <= 64 ? 64u : t.n <= 128 ? 128u : 256u;
   if (tid == 0) {
     for (int s = 0; s < S; s++) {
-      mbar_init(&full_bar[s], PRODUCERS);
+      mbar_init(&full_bar[s], PRODUCERS / 32);
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&done_bar, 1);
@@ -225,22 +247,48 @@ NGS_DEV void run_tile(const TileShape& t, uint8_t* smem, Fill& fill, Store& stor
   const uint32_t tmem = tmem_slot;
 
   if (tid < PRODUCERS) {
-    // producers: fill the ring of stages
-    for (int s = 0; s < t.steps; s++) {
-      const int st = s % S;
-      if (s >= S && !mbar_wait(&empty_bar[st], (uint32_t)((s / S) - 1) & 1u, &abort_flag)) break;
+    // producers: fill the ring of stages (the ring position and its round are counted along: a division
+    // by the stage count costs more instructions than a stage's copies)
+    auto hand_over = [&](int st) {
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[st]);
+    };
+    int s = 0, st = 0;
+    uint32_t parity = 1u;                        // of the round before this one
+    for (; s < t.steps; s++) {
+      const bool go = s < S || mbar_wait(&empty_bar[st], parity, &abort_flag);
+      if (!__all_sync(0xffffffffu, go)) break;
       uint8_t* a = smem + (size_t)st * t.stage_bytes;
       const int valid = fill(s, a, a + A_BYTES, tid);
       if (tid == 0) ksteps_of[st] = (valid + UK - 1) / UK;
-      fence_async_smem();
-      mbar_arrive(&full_bar[st]);
+      if constexpr (ASYNC) {
+        cp_async_commit();
+        if (s >= AHEAD) {
+          cp_async_wait<AHEAD>();
+          hand_over(st >= AHEAD ? st - AHEAD : st - AHEAD + S);
+        }
+      } else {
+        hand_over(st);
+      }
+      if (++st == S) {
+        st = 0;
+        parity ^= 1u;
+      }
+    }
+    if constexpr (ASYNC) {
+      // the last stages; after an abort the copies still land before the shared memory is given up
+      cp_async_wait<0>();
+      if (s == t.steps)
+        for (int r = max(0, s - AHEAD); r < s; r++) hand_over(r % S);
     }
   } else if (lane == 0) {
     // one thread issues the MMAs of every stage, then commits the stage back to the producers
     const uint32_t idesc = mn_major ? f16_idesc_mn(BM, t.n, bf16) : f16_idesc(BM, t.n, bf16);
+    int st = 0;
+    uint32_t parity = 0u;
     for (int s = 0; s < t.steps; s++) {
-      const int st = s % S;
-      if (!mbar_wait(&full_bar[st], (uint32_t)(s / S) & 1u, &abort_flag)) break;
+      if (!mbar_wait(&full_bar[st], parity, &abort_flag)) break;
       tc_fence_after();
       const uint32_t a = smem_u32(smem + (size_t)st * t.stage_bytes), b = a + A_BYTES;
       const int ks = ksteps_of[st];
@@ -250,6 +298,10 @@ NGS_DEV void run_tile(const TileShape& t, uint8_t* smem, Fill& fill, Store& stor
                  mn_major ? mnmajor_sw128_desc(b + kk * 2048) : kmajor_sw128_desc(b + kk * 32), idesc,
                  (s > 0 || kk > 0) ? 1u : 0u);
       umma_commit(&empty_bar[st]);
+      if (++st == S) {
+        st = 0;
+        parity ^= 1u;
+      }
     }
     umma_commit(&done_bar);        // arrives once everything issued above has completed
   }
@@ -317,6 +369,7 @@ struct GatherGemm {
   int64_t n_src;
   int kdim;
   const int32_t* table;
+  int64_t row_stride, k_stride;   // of the table: entry (row, k) at row * row_stride + k * k_stride
   int64_t n_rows;
   int K;
   const uint16_t* bt;
@@ -343,9 +396,14 @@ __global__ void __launch_bounds__(conv::THREADS, 1) conv_gather_gemm_kernel(cons
   // the offsets with at least one pair in this tile (empty offsets cost nothing)
   if (tid < KMAX / 32) act_mask[tid] = 0u;
   __syncthreads();
-  if (tid < BM && r0 + tid < g.n_rows)
-    for (int k = 0; k < g.K; k++)
-      if (__ldg(g.table + (r0 + tid) * g.K + k) >= 0) atomicOr(&act_mask[k >> 5], 1u << (k & 31));
+  if (tid < BM && r0 + tid < g.n_rows) {
+    const int32_t* t0 = g.table + (r0 + tid) * g.row_stride;
+#pragma unroll 9
+    for (int k = 0; k < g.K; k++) {
+      const unsigned any = __ballot_sync(__activemask(), __ldg(t0 + k * g.k_stride) >= 0);
+      if (any && (tid & 31) == 0) atomicOr(&act_mask[k >> 5], 1u << (k & 31));
+    }
+  }
   __syncthreads();
   if (tid == 0) {
     int c = 0;
@@ -357,33 +415,54 @@ __global__ void __launch_bounds__(conv::THREADS, 1) conv_gather_gemm_kernel(cons
   const int nchunks = (g.kdim + BK - 1) / BK;
   TileShape t{n_act * nchunks, N, g.stages, g.stage_bytes};
 
-  // two producers per tile row, four 16-byte chunks each; B rows spread over all producers
+  // eight producers per tile row, one 16-byte chunk each (a row's 128 bytes in one request), four rows
+  // per producer; the rows' table entries are read one offset ahead.  B rows likewise.  The bound is the
+  // producers' instructions (18 warps an SM, 9 cycles from one to the next), not the memory: 1.3M rows of
+  // 64 -> 64 channels took 1.67 ms with loads through registers, 1.64 with asynchronous copies alone,
+  // 1.31 once the ring's divisions and the variable-size form of the copies were gone.
+  const int prow = tid >> 3, pchunk = tid & 7;
+  const uint32_t at = sw128(prow, pchunk);            // 32 rows further on: 4 KB
+  const int32_t* const trow = g.table + (r0 + prow) * g.row_stride;
+  const int left = (int)min((int64_t)BM, g.n_rows - r0) - prow;
+  const unsigned n_src = (unsigned)g.n_src;
+  const int kdim = g.kdim;
+  auto entries = [&](int i, int32_t (&src)[4]) {
+    const int32_t* tk = trow + act_list[i] * g.k_stride;
+#pragma unroll
+    for (int j = 0; j < 4; j++) src[j] = 32 * j < left ? __ldg(tk + 32 * j * g.row_stride) : -1;
+  };
+  int32_t src[4] = {-1, -1, -1, -1}, next[4] = {-1, -1, -1, -1};
+  int active = 0, c0 = 0;                             // the step's place in act_list and its first channel
+  if (tid < PRODUCERS && t.steps > 0) entries(0, src);
   auto fill = [&](int s, uint8_t* a, uint8_t* b, int p) -> int {
-    const int k = act_list[s / nchunks];
-    const int c0 = (s % nchunks) * BK;
-    const int row = p >> 1, half = p & 1;
-    int32_t src = -1;
-    if (r0 + row < g.n_rows) src = __ldg(g.table + (r0 + row) * g.K + k);
-    const bool have = src >= 0 && src < g.n_src;
-    uint4 v[4];
+    const int k = act_list[active], e = c0 + pchunk * 8, valid = min(BK, kdim - c0);
+    const bool in = e < kdim;
+    if (c0 == 0 && active + 1 < n_act) entries(active + 1, next);
+    const uint16_t* xe = g.x + e;
+    const uint32_t sa = smem_u32(a), sb = smem_u32(b);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int e = c0 + (half * 4 + j) * 8;
-      v[j] = (have && e < g.kdim) ? ldg16(g.x + (int64_t)src * g.kdim + e) : make_uint4(0, 0, 0, 0);
+      const bool have = in && (unsigned)src[j] < n_src;
+      cp_async16(sa + at + j * 4096, have ? xe + (int64_t)src[j] * kdim : g.x, have);
     }
+    const uint16_t* bk = g.bt + ((int64_t)k * g.ncols + n0 + prow) * kdim;
+    for (int n = prow; n < N; n += 32) {
+      cp_async16(sb + at + (n - prow) * 128, in ? bk + e : g.bt, in);
+      bk += 32 * kdim;
+    }
+    c0 += BK;
+    if (c0 >= kdim) {
+      c0 = 0;
+      active++;
 #pragma unroll
-    for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(a + sw128(row, half * 4 + j)) = v[j];
-    for (int idx = p; idx < N * 8; idx += PRODUCERS) {
-      const int n = idx >> 3, c = idx & 7, e = c0 + c * 8;
-      const uint4 w = e < g.kdim ? ldg16(g.bt + ((int64_t)k * g.ncols + n0 + n) * g.kdim + e) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(b + sw128(n, c)) = w;
+      for (int j = 0; j < 4; j++) src[j] = next[j];
     }
-    return min(BK, g.kdim - c0);
+    return valid;
   };
   auto store = [&](int row, int col, const float (&v)[16]) {
     if (r0 + row < g.n_rows) st16_row(g.out, g.out_f32 != 0, g.bf16, (r0 + row) * g.ncols + n0 + col, v);
   };
-  run_tile(t, smem, fill, store, g.bf16, g.error);
+  run_tile<true>(t, smem, fill, store, g.bf16, g.error);
 }
 
 // ----------------------------------------------------------------------------- weight gradient
@@ -414,6 +493,7 @@ __global__ void __launch_bounds__(conv::THREADS, 1) conv_wgrad_kernel(const __gr
   using namespace conv;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int tid = threadIdx.x;
   const int split = blockIdx.x, k = blockIdx.y;
   const int m0 = (blockIdx.z % g.m_tiles) * BM, n0 = (blockIdx.z / g.m_tiles) * 256;
   const int N = min(256, g.cout - n0);
@@ -453,30 +533,51 @@ __global__ void __launch_bounds__(conv::THREADS, 1) conv_wgrad_kernel(const __gr
     return (int)min((int64_t)BK, p_count - pc);
   };
   // MN-major form: the stage's K index is the pair, each 128-byte row 64 consecutive channels of one
-  // pair, so a producer copies 16-byte pieces of its pair's rows as they are (no transposition)
-  auto fill_mn = [&](int s, uint8_t* a, uint8_t* b, int p) -> int {
-    const int64_t pc = (c_begin + s) * BK;
-    const int kk = p & 63, q = p >> 6;
-    const int64_t pair = pc + kk;
-    int32_t xi = -1, yo = -1;
-    if (pair < p_count) {
-      xi = __ldg(g.nbmaps + 2 * (p_begin + pair) + g.in_col);
-      yo = __ldg(g.nbmaps + 2 * (p_begin + pair) + 1 - g.in_col);
-    }
-    const bool hx = xi >= 0 && xi < g.n_in, hy = yo >= 0 && yo < g.n_out;
+  // pair, so a producer copies 16-byte pieces of its pairs' rows as they are (no transposition): eight
+  // producers per 128 bytes, two pairs each.  Channels past cin are zeroed once, before the first step.
+  const int prow = tid >> 3, pchunk = tid & 7;
+  const int a_atoms = min(2, (g.cin - m0) / 64), b_atoms = N / 64;
+  auto pairs = [&](int s, int32_t (&xi)[2], int32_t (&yo)[2]) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {                    // A: 16 chunks of 8 channels, 4 per quarter
-      const int c = q * 4 + j, ch = m0 + c * 8;
-      const uint4 v = (hx && ch < g.cin) ? ldg16(g.x + (int64_t)xi * g.cin + ch) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(a + (c >> 3) * MN_ATOM_BYTES + sw128(kk, c & 7)) = v;
+    for (int j = 0; j < 2; j++) {
+      const int64_t pair = (c_begin + s) * BK + prow + 32 * j;
+      xi[j] = yo[j] = -1;
+      if (pair < p_count) {
+        xi[j] = __ldg(g.nbmaps + 2 * (p_begin + pair) + g.in_col);
+        yo[j] = __ldg(g.nbmaps + 2 * (p_begin + pair) + 1 - g.in_col);
+      }
     }
-    const int per = N / 32;                          // B: N / 8 chunks, a quarter each
-    for (int j = 0; j < per; j++) {
-      const int c = q * per + j, ch = n0 + c * 8;
-      const uint4 v = hy ? ldg16(g.gy + (int64_t)yo * g.cout + ch) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(b + (c >> 3) * MN_ATOM_BYTES + sw128(kk, c & 7)) = v;
+  };
+  int32_t nx[2] = {-1, -1}, ny[2] = {-1, -1};
+  const uint32_t at = sw128(prow, pchunk);
+  const unsigned n_in = (unsigned)g.n_in, n_out = (unsigned)g.n_out;
+  const uint16_t *x0 = g.x + m0 + pchunk * 8, *y0 = g.gy + n0 + pchunk * 8;
+  if (g.mn) {
+    if (a_atoms < 2)
+      for (int st = 0; st < g.stages; st++)
+        for (int i = tid; i < (int)MN_ATOM_BYTES / 16; i += THREADS)
+          *reinterpret_cast<uint4*>(smem + (size_t)st * g.stage_bytes + MN_ATOM_BYTES + i * 16) = make_uint4(0, 0, 0, 0);
+    fence_async_smem();
+    if (tid < PRODUCERS && t.steps > 0) pairs(0, nx, ny);
+  }
+  auto fill_mn = [&](int s, uint8_t* a, uint8_t* b, int p) -> int {
+    int32_t xi[2], yo[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      xi[j] = nx[j];
+      yo[j] = ny[j];
     }
-    return (int)min((int64_t)BK, p_count - pc);
+    const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+    if (s + 1 < t.steps) pairs(s + 1, nx, ny);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const bool hx = (unsigned)xi[j] < n_in, hy = (unsigned)yo[j] < n_out;
+      const uint16_t* xr = hx ? x0 + (int64_t)xi[j] * g.cin : g.x;
+      const uint16_t* yr = hy ? y0 + (int64_t)yo[j] * g.cout : g.gy;
+      for (int c = 0; c < a_atoms; c++) cp_async16(sa + c * MN_ATOM_BYTES + at + j * 4096, xr + (hx ? c * 64 : 0), hx);
+      for (int c = 0; c < b_atoms; c++) cp_async16(sb + c * MN_ATOM_BYTES + at + j * 4096, yr + (hy ? c * 64 : 0), hy);
+    }
+    return (int)min((int64_t)BK, p_count - (c_begin + s) * BK);
   };
   float* part = g.part + ((int64_t)k * g.splits + split) * g.cin * g.cout;
   auto store = [&](int row, int col, const float (&v)[16]) {
@@ -486,8 +587,8 @@ __global__ void __launch_bounds__(conv::THREADS, 1) conv_wgrad_kernel(const __gr
       for (int j = 0; j < 4; j++) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
   };
-  if (g.mn) run_tile(t, smem, fill_mn, store, g.bf16, g.error, true);
-  else run_tile(t, smem, fill, store, g.bf16, g.error);
+  if (g.mn) run_tile<true>(t, smem, fill_mn, store, g.bf16, g.error, true);
+  else run_tile<false>(t, smem, fill, store, g.bf16, g.error);
 }
 
 // grad_w[k, c, n] = sum over splits (in order) of part[k, split, c, n]; FP32 or 16-bit out.
@@ -549,8 +650,8 @@ NGS_DEV bool finite4(float4 v) { return isfinite(v.x) && isfinite(v.y) && isfini
 // thread per output that reads its rows and weights for itself.
 template <typename T, int BM, int BN, int CK>
 __global__ void __launch_bounds__(BM* BN / 16) conv_gather_gemm_simt_kernel(
-    const T* __restrict__ x, int64_t n_src, int kdim, const int32_t* __restrict__ table, int64_t n_rows, int K,
-    const T* __restrict__ bt, int ncols, void* out, int out_f32, int vec) {
+    const T* __restrict__ x, int64_t n_src, int kdim, const int32_t* __restrict__ table, int64_t row_stride,
+    int64_t k_stride, int64_t n_rows, int K, const T* __restrict__ bt, int ncols, void* out, int out_f32, int vec) {
   constexpr int NT = BM * BN / 16;
   constexpr int NA = BM * CK / 4 / NT, NB = (BN * CK / 4 + NT - 1) / NT;
   __shared__ __align__(16) float As[CK][BM + 4];
@@ -563,9 +664,10 @@ __global__ void __launch_bounds__(BM* BN / 16) conv_gather_gemm_simt_kernel(
   for (int k = t; k < (conv::KMAX + 31) / 32; k += NT) s_any[k] = 0u;
   __syncthreads();
   const int rows = (int)min((int64_t)BM, n_rows - r0);
-  for (int e = t; e < rows * K; e += NT) {
-    const int32_t src = table[r0 * K + e];
-    const int k = e % K;
+  for (int e = t; e < BM * K; e += NT) {
+    const int row = e % BM, k = e / BM;
+    if (row >= rows) continue;
+    const int32_t src = table[(r0 + row) * row_stride + k * k_stride];
     if (src >= 0 && src < n_src) atomicOr(&s_any[k >> 5], 1u << (k & 31));
   }
   __syncthreads();
@@ -580,7 +682,7 @@ __global__ void __launch_bounds__(BM* BN / 16) conv_gather_gemm_simt_kernel(
 #pragma unroll
     for (int j = 0; j < NA; j++) {
       const int e = t + j * NT, row = e % BM, c = c0 + e / BM * 4;
-      const int32_t src = row < rows ? __ldg(table + (r0 + row) * K + k) : -1;
+      const int32_t src = row < rows ? __ldg(table + (r0 + row) * row_stride + k * k_stride) : -1;
       const bool ok = src >= 0 && src < n_src;
       if (j == 0) va = ok;                            // thread t < BM stages row t first
       ra[j] = ok ? load4<T>(x + (int64_t)src * kdim, c, kdim, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -792,28 +894,28 @@ void tile_plan(int n, int& stages, uint32_t& stage_bytes, size_t& smem) {
 // Column tile of the CUDA-core kernels: the smallest of 16, 32 and 64 that holds the columns (a narrower
 // tile than the columns need would gather the rows once more, a wider one multiplies zeros).
 template <typename T, int BM, int BN>
-int simt_gemm_tile(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K, const void* bt,
-                   int ncols, void* out, int out_f32, cudaStream_t st) {
-  const dim3 grid((unsigned)((n_rows + BM - 1) / BM), (unsigned)((ncols + BN - 1) / BN));
-  ngs_count_launch();
+int simt_gemm_tile(const GatherGemm& g, cudaStream_t st) {
+  const dim3 grid((unsigned)((g.n_rows + BM - 1) / BM), (unsigned)((g.ncols + BN - 1) / BN));
+  const T* x = reinterpret_cast<const T*>(g.x);
+  const T* bt = reinterpret_cast<const T*>(g.bt);
   // slices of 32 channels where there are more than 16: half the stages, and a stage is a round trip
-  const int vec = kdim % 4 == 0 && aligned16(x) && aligned16(bt);
-  if (kdim <= 16)
+  const int vec = g.kdim % 4 == 0 && aligned16(x) && aligned16(bt);
+  ngs_count_launch();
+  if (g.kdim <= 16)
     conv_gather_gemm_simt_kernel<T, BM, BN, 16><<<grid, BM * BN / 16, 0, st>>>(
-        static_cast<const T*>(x), n_src, kdim, table, n_rows, K, static_cast<const T*>(bt), ncols, out, out_f32, vec);
+        x, g.n_src, g.kdim, g.table, g.row_stride, g.k_stride, g.n_rows, g.K, bt, g.ncols, g.out, g.out_f32, vec);
   else
     conv_gather_gemm_simt_kernel<T, BM, BN, 32><<<grid, BM * BN / 16, 0, st>>>(
-        static_cast<const T*>(x), n_src, kdim, table, n_rows, K, static_cast<const T*>(bt), ncols, out, out_f32, vec);
+        x, g.n_src, g.kdim, g.table, g.row_stride, g.k_stride, g.n_rows, g.K, bt, g.ncols, g.out, g.out_f32, vec);
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }
 
 template <typename T>
-int simt_gemm(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K, const void* bt,
-              int ncols, void* out, int out_f32, cudaStream_t st) {
-  if (ncols <= 16) return simt_gemm_tile<T, 64, 16>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
-  if (ncols <= 32) return simt_gemm_tile<T, 64, 32>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
-  return simt_gemm_tile<T, 64, 64>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
+int simt_gemm(const GatherGemm& g, cudaStream_t st) {
+  if (g.ncols <= 16) return simt_gemm_tile<T, 64, 16>(g, st);
+  if (g.ncols <= 32) return simt_gemm_tile<T, 64, 32>(g, st);
+  return simt_gemm_tile<T, 64, 64>(g, st);
 }
 
 // Splits of the pairs: at least 512 pairs each (CUDA cores) or 2,048 (tensor cores), at most 64.
@@ -884,32 +986,33 @@ extern "C" int ngs_conv_tensor_core_ok(int kdim, int ncols, int dtype) {
   return (dtype == NGS_F16 || dtype == NGS_BF16) && kdim >= 8 && kdim % 8 == 0 && ncols >= 16 && ncols % 16 == 0;
 }
 
-extern "C" int ngs_conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K,
-                                    const void* bt, int ncols, int dtype, void* out, int out_f32, int* error_dev,
-                                    ngs_stream s) {
+static int conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t row_stride,
+                            int64_t k_stride, int64_t n_rows, int K, const void* bt, int ncols, int dtype, void* out,
+                            int out_f32, int* error_dev, cudaStream_t st) {
   if (n_src < 0 || n_rows < 0 || kdim < 1 || ncols < 1 || K < 1 || K > conv::KMAX || dtype < NGS_F16 ||
       dtype > NGS_F32 || (n_rows > 0 && (!table || !out || !bt)) || (n_src > 0 && !x) || !error_dev)
     return NGS_ERR_INVALID_ARG;
   if (n_rows == 0) return NGS_OK;
-  cudaStream_t st = (cudaStream_t)s;
-  if (!ngs_conv_tensor_core_ok(kdim, ncols, dtype) || !aligned16(x) || !aligned16(bt) || !aligned16(out)) {
-    if (dtype == NGS_F32) return simt_gemm<float>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, 1, st);
-    if (dtype == NGS_BF16) return simt_gemm<__nv_bfloat16>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
-    return simt_gemm<__half>(x, n_src, kdim, table, n_rows, K, bt, ncols, out, out_f32, st);
-  }
   GatherGemm g{};
-  g.x = static_cast<const uint16_t*>(x);
+  g.x = static_cast<const uint16_t*>(n_src > 0 ? x : bt);   // a valid address also where every row is missing
   g.n_src = n_src;
   g.kdim = kdim;
   g.table = table;
+  g.row_stride = row_stride;
+  g.k_stride = k_stride;
   g.n_rows = n_rows;
   g.K = K;
   g.bt = static_cast<const uint16_t*>(bt);
   g.ncols = ncols;
   g.out = out;
-  g.out_f32 = out_f32;
+  g.out_f32 = out_f32 || dtype == NGS_F32;
   g.bf16 = dtype == NGS_BF16;
   g.error = error_dev;
+  if (!ngs_conv_tensor_core_ok(kdim, ncols, dtype) || !aligned16(x) || !aligned16(bt) || !aligned16(out)) {
+    if (dtype == NGS_F32) return simt_gemm<float>(g, st);
+    if (dtype == NGS_BF16) return simt_gemm<__nv_bfloat16>(g, st);
+    return simt_gemm<__half>(g, st);
+  }
   size_t smem = 0;
   tile_plan(ncols < 256 ? ncols : 256, g.stages, g.stage_bytes, smem);
   if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -920,6 +1023,20 @@ extern "C" int ngs_conv_gather_gemm(const void* x, int64_t n_src, int kdim, cons
   conv_gather_gemm_kernel<<<grid, conv::THREADS, smem, st>>>(g);
   NGS_CHECK_LAUNCH();
   return NGS_OK;
+}
+
+extern "C" int ngs_conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_t* table, int64_t n_rows, int K,
+                                    const void* bt, int ncols, int dtype, void* out, int out_f32, int* error_dev,
+                                    ngs_stream s) {
+  return conv_gather_gemm(x, n_src, kdim, table, K, 1, n_rows, K, bt, ncols, dtype, out, out_f32, error_dev,
+                          (cudaStream_t)s);
+}
+
+extern "C" int ngs_conv_gather_gemm_kmajor(const void* x, int64_t n_src, int kdim, const int32_t* table,
+                                           int64_t n_rows, int K, const void* bt, int ncols, int dtype, void* out,
+                                           int out_f32, int* error_dev, ngs_stream s) {
+  return conv_gather_gemm(x, n_src, kdim, table, 1, n_rows, n_rows, K, bt, ncols, dtype, out, out_f32, error_dev,
+                          (cudaStream_t)s);
 }
 
 extern "C" size_t ngs_conv_weight_grad_ws_bytes(int K, int cin, int cout, int64_t max_pairs) {
@@ -950,8 +1067,8 @@ extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const 
   const size_t need = (size_t)K * splits * cin * cout * sizeof(float);
   if (!ws || ws_bytes < need) return NGS_ERR_OOM;
   WeightGrad g{};
-  g.x = static_cast<const uint16_t*>(x);
-  g.gy = static_cast<const uint16_t*>(gy);
+  g.x = static_cast<const uint16_t*>(n_in > 0 ? x : grad_w);     // a valid address also where every pair is skipped
+  g.gy = static_cast<const uint16_t*>(n_out > 0 ? gy : grad_w);
   g.n_in = n_in;
   g.n_out = n_out;
   g.cin = cin;

@@ -297,8 +297,8 @@ def _offset_starts(neighbor_offset, K: int, device):
 
 
 def _conv_table(neighbor_map, starts, K, key_col, n_rows, mid):
-    table = torch.empty((n_rows, K), dtype=torch.int32, device=neighbor_map.device)
-    L.call("ngs_conv_table", L.ptr(neighbor_map), L.ptr(starts), K, key_col, n_rows, mid, L.ptr(table), L.stream())
+    table = torch.empty((K, n_rows), dtype=torch.int32, device=neighbor_map.device)
+    L.call("ngs_conv_table_kmajor", L.ptr(neighbor_map), L.ptr(starts), K, key_col, n_rows, mid, L.ptr(table), L.stream())
     return table
 
 
@@ -306,7 +306,7 @@ def _gather_gemm(x, table, bt, ncols, out):
     err = torch.zeros(1, dtype=torch.int32, device=x.device)
     dt = _conv_dtype(x)
     out_f32 = int(out.dtype == torch.float32)
-    L.call("ngs_conv_gather_gemm", L.ptr(x), x.shape[0], x.shape[1], L.ptr(table), table.shape[0], table.shape[1],
+    L.call("ngs_conv_gather_gemm_kmajor", L.ptr(x), x.shape[0], x.shape[1], L.ptr(table), table.shape[1], table.shape[0],
            L.ptr(bt), ncols, dt, L.ptr(out), out_f32, L.ptr(err), L.stream())
     return err
 

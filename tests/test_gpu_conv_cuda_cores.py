@@ -68,3 +68,21 @@ def test_non_finite_weights_reach_only_the_rows_with_a_pair(bad):
     hit[maps[at:at + int(sizes[3]), 1].long()] = True
     assert torch.equal(~torch.isfinite(y[:, 11]), hit) and torch.isfinite(y[:, :11]).all() and torch.isfinite(y[:, 12:]).all()
 
+
+@pytest.mark.parametrize("n_in,n_out", [(70, 127), (300, 128), (513, 400)])
+@pytest.mark.parametrize("cin,cout,dtype", [(16, 24, torch.float32), (64, 64, torch.float16), (40, 272, torch.bfloat16)])
+def test_both_table_layouts_give_the_same_bits(n_in, n_out, cin, cout, dtype):
+    """Tables with the row outermost (ngs_conv_table) and with the offset outermost (.._kmajor)."""
+    from jspsr import _lib as L, ext
+    K = 8
+    maps, sizes = layer(n_in, n_out, K, n_out)
+    starts, _ = ext._offset_starts(sizes, K, DEV)
+    x, w = torch.randn(n_in, cin, device=DEV).to(dtype), torch.randn(K, cout, cin, device=DEV).to(dtype)
+    y = [torch.empty(n_out, cout, device=DEV, dtype=dtype) for _ in range(2)]
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    tables = [torch.empty(n_out, K, dtype=torch.int32, device=DEV), torch.empty(K, n_out, dtype=torch.int32, device=DEV)]
+    for t, out, end in zip(tables, y, ("", "_kmajor")):
+        L.call("ngs_conv_table" + end, L.ptr(maps), L.ptr(starts), K, 1, n_out, -1, L.ptr(t), L.stream())
+        L.call("ngs_conv_gather_gemm" + end, L.ptr(x), n_in, cin, L.ptr(t), n_out, K, L.ptr(w), cout, ext._conv_dtype(x),
+               L.ptr(out), int(dtype == torch.float32), L.ptr(err), L.stream())
+    assert torch.equal(tables[0].T, tables[1]) and torch.equal(y[0], y[1]) and int(err) == 0
