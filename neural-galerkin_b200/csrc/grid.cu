@@ -350,26 +350,47 @@ extern "C" int ngs_density_eval(ngs_grid g, const float* xyz, int64_t n, float i
   return NGS_OK;
 }
 
-__global__ void point_basis_kernel(ngs_grid g, const float* __restrict__ xyz, int64_t n, float inv_vs, double vs,
-                                   int32_t* __restrict__ rows, float* __restrict__ phi) {
-  for (int64_t p = ngs_gtid(); p < n; p += ngs_gstride()) {
-    const PointNbr nb = point_nbr(xyz + p * 3, inv_vs, vs, g.stride);
-    float bx[3], by[3], bz[3];
+// A block's 128 points are staged in shared memory, so that the [n, 27] arrays are written in order (27
+// words apart, every store of a thread-per-point loop is a sector of its own), with the cells of a run along
+// z looked up together.  300,000 points, 4 levels: 0.12 ms against 0.57; 5M points, 11 levels: 4.0 against 24.7.
+constexpr int BASIS_POINTS = 128;
+__global__ void __launch_bounds__(BASIS_POINTS) point_basis_kernel(ngs_grid g, const float* __restrict__ xyz,
+                                                                   int64_t n, float inv_vs, double vs,
+                                                                   int32_t* __restrict__ rows, float* __restrict__ phi) {
+  __shared__ int32_t s_row[BASIS_POINTS * 27];
+  __shared__ float s_phi[BASIS_POINTS * 27];
+  for (int64_t p0 = (int64_t)blockIdx.x * BASIS_POINTS; p0 < n; p0 += (int64_t)gridDim.x * BASIS_POINTS) {
+    const int64_t p = p0 + threadIdx.x;
+    if (p < n) {
+      const PointNbr nb = point_nbr(xyz + p * 3, inv_vs, vs, g.stride);
+      float bx[3], by[3], bz[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      bx[k] = bspline(nb.rel[0][k]);
-      by[k] = bspline(nb.rel[1][k]);
-      bz[k] = bspline(nb.rel[2][k]);
-    }
-    for (int kx = 0; kx < 3; kx++)
-      for (int ky = 0; ky < 3; ky++)
-        for (int kz = 0; kz < 3; kz++) {
-          const int o = kx * 9 + ky * 3 + kz;
-          const int64_t r = grid_row(g, nb.q[0] + (kx - 1) * g.stride, nb.q[1] + (ky - 1) * g.stride,
-                                     nb.q[2] + (kz - 1) * g.stride);
-          rows[p * 27 + o] = (int32_t)r;
-          phi[p * 27 + o] = r >= 0 ? bx[kx] * by[ky] * bz[kz] : 0.f;
+      for (int k = 0; k < 3; k++) {
+        bx[k] = bspline(nb.rel[0][k]);
+        by[k] = bspline(nb.rel[1][k]);
+        bz[k] = bspline(nb.rel[2][k]);
+      }
+#pragma unroll
+      for (int kx = 0; kx < 3; kx++)
+#pragma unroll
+        for (int ky = 0; ky < 3; ky++) {
+          int32_t r[3];
+          grid_rows_zrun<3>(g, nb.q[0] + (kx - 1) * g.stride, nb.q[1] + (ky - 1) * g.stride, nb.q[2] - g.stride, r);
+#pragma unroll
+          for (int kz = 0; kz < 3; kz++) {
+            const int o = threadIdx.x * 27 + kx * 9 + ky * 3 + kz;
+            s_row[o] = r[kz];
+            s_phi[o] = r[kz] >= 0 ? bx[kx] * by[ky] * bz[kz] : 0.f;
+          }
         }
+    }
+    __syncthreads();
+    const int m = (int)min((int64_t)BASIS_POINTS, n - p0) * 27;
+    for (int e = threadIdx.x; e < m; e += BASIS_POINTS) {
+      rows[p0 * 27 + e] = s_row[e];
+      phi[p0 * 27 + e] = s_phi[e];
+    }
+    __syncthreads();
   }
 }
 
@@ -377,11 +398,13 @@ extern "C" int ngs_point_basis(ngs_grid g, const float* xyz, int64_t n, float in
                                float* phi, ngs_stream s) {
   if (!grid_ok(g) || n < 0 || (n > 0 && (!xyz || !rows || !phi))) return NGS_ERR_INVALID_ARG;
   if (n == 0) return NGS_OK;
-  { ngs_count_launch(); point_basis_kernel<<<ngs_blocks(n, 128), 128, 0, (cudaStream_t)s>>>(g, xyz, n, inv_vs, vs, rows, phi); }
+  { ngs_count_launch(); point_basis_kernel<<<ngs_blocks(n, BASIS_POINTS), BASIS_POINTS, 0, (cudaStream_t)s>>>(g, xyz, n, inv_vs, vs, rows, phi); }
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }
 
+// (Staging the [n, 27] arrays through shared memory, as point_basis_kernel does, was slower: 45 against 31 us
+// for 300,000 points -- the reads of neighbouring threads meet in L1.)
 __global__ void point_field_kernel(const int32_t* __restrict__ rows, const float* __restrict__ phi, int64_t n,
                                    const float* __restrict__ x, float* __restrict__ out, int accumulate) {
   for (int64_t p = ngs_gtid(); p < n; p += ngs_gstride()) {

@@ -567,7 +567,9 @@ class Reconstruction(DualMesher):
         return out
 
     # ------------------------------------------------------------------ RHS + solve
-    def _rhs(self, d):
+    def _rhs(self, d, coarse_field=None):
+        """Right-hand side of level d.  ``coarse_field``: the coarser levels' field at the points, where the
+        caller sums it up level by level; formed here otherwise."""
         st = L.stream()
         lv = self.levels[d]
         rhs = torch.zeros(lv.n, dtype=torch.float64, device=self.dev)
@@ -586,11 +588,11 @@ class Reconstruction(DualMesher):
         coarser = list(range(self.depth - 1, d, -1))
         if coarser:
             if self.alpha > 0:
-                fieldp = torch.zeros(self.n, dtype=torch.float32, device=self.dev)
-                for dd in coarser:
-                    lc = self.levels[dd]
-                    L.call("ngs_point_field", L.ptr(lc.rows), L.ptr(lc.phi), self.n, L.ptr(lc.x32), L.ptr(fieldp), 1, st)
-                self._screen_rhs(lv, fieldp, -sf * self.alpha, rhs)
+                if coarse_field is None:
+                    coarse_field = torch.zeros(self.n, dtype=torch.float32, device=self.dev)
+                    for dd in coarser:
+                        self._add_field(self.levels[dd], coarse_field)
+                self._screen_rhs(lv, coarse_field, -sf * self.alpha, rhs)
             for dd in coarser:
                 lc = self.levels[dd]
                 tc = L.device_table(("corr_c", lv.stride, lc.stride),
@@ -601,6 +603,10 @@ class Reconstruction(DualMesher):
                        L.ptr(tc), L.ptr(tg), tc.numel(), L.ptr(rhs), st)
         lv.rhs = rhs
         return rhs
+
+    def _add_field(self, lv: Level, field: torch.Tensor):
+        """field += the level's solution at the points."""
+        L.call("ngs_point_field", L.ptr(lv.rows), L.ptr(lv.phi), self.n, L.ptr(lv.x32), L.ptr(field), 1, L.stream())
 
     def _screen_rhs(self, lv: Level, val, scale: float, rhs: torch.Tensor):
         """rhs += scale * sum over the level's points of phi * (val[point] or 1): gathered per row from the
@@ -725,8 +731,15 @@ class Reconstruction(DualMesher):
 
     def solve(self):
         """Coarse-to-fine solve (reconstructor.py:122-189)."""
+        field = None
+        if self.alpha > 0 and self.depth > 1:
+            # the solved levels' field at the points, one level added after each solve (not all of them
+            # again for every finer level)
+            field = torch.zeros(self.n, dtype=torch.float32, device=self.dev)
         for d in range(self.depth - 1, -1, -1):
-            self._rhs(d)
+            if field is not None and d < self.depth - 1:
+                self._add_field(self.levels[d + 1], field)
+            self._rhs(d, field)
             self._mark(f"rhs{d}")
             self._solve_level(self.levels[d], d)
             self._mark(f"pcg{d}")
