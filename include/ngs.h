@@ -526,6 +526,28 @@ int ngs_dual_mc_indices_grid(ngs_grid dual, const int32_t* primal_base, int64_t 
                              int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s);
 int ngs_dual_mc_indices_hash(const ngs_hash_table* dual, const int32_t* primal_base, int64_t n_primal, int stride,
                              int depth, int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s);
+/* Two-level rank bitmap of dual centres, for boxes too large for a plain ngs_grid: `outer` is an ngs_grid of
+ * stride 1 over (x, y, z / 64) -- origin the box's corner, dims[2] the number of 64-cell words along z --
+ * and `inner` holds only the words that contain a cell, 16 bytes each as ngs_grid.words, in the order of
+ * the outer grid's ranks; `blocks` (ngs_grid2_block_bytes, zeroed) has a bit per 32 x 32 columns x word.
+ * Build: mark with pass 0, ngs_grid_finalize the outer grid (its count is the number of inner words),
+ * provide `inner` zeroed, mark with pass 1, and finalize `inner` (as an ngs_grid of {words, 1, 64} cells).
+ * Rows are ranks in (x, y, z) order, as a plain grid's.  mark_cell_corners / mark_coords mark what
+ * ngs_grid_mark_cell_corners / ngs_grid_mark_coords mark; the indices functions fill acc and cnt as the ones
+ * on a plain grid do (cell bases must be multiples of the stride). */
+typedef struct ngs_grid2 {
+  ngs_grid outer;
+  void* inner;
+  uint32_t* blocks;
+} ngs_grid2;
+size_t ngs_grid2_block_bytes(ngs_grid outer);
+int ngs_grid2_mark_cell_corners(ngs_grid2 g, int pass, const int32_t* cells, int64_t n, int stride, ngs_stream s);
+int ngs_grid2_mark_coords(ngs_grid2 g, int pass, const int32_t* coords, int64_t n, const int32_t* offsets, int n_off,
+                          int offset_scale, ngs_stream s);
+int ngs_dual_mc_indices_grid2(ngs_grid2 dual, const int32_t* primal_base, int64_t n_primal, int stride, int depth,
+                              int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s);
+int ngs_dual_mc_indices_cells2(ngs_grid2 dual, const int32_t* cells, int64_t n_cells, int depth, int64_t idx_base,
+                               int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s);
 /* The same accumulation for level-0 leaf cells (cell stride 1, n_up = 2) given as cells, not as
  * expanded samples: the 8 samples of cell i have ids idx_base + 8 i + e (ngs_expand_cells order);
  * each of a cell's 27 sample corners is looked up once.  dual must have stride 1. */

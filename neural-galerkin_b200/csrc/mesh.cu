@@ -1,6 +1,7 @@
 // Multi-level dual marching cubes (jspsr/core/reconstructor.py:296-397,
 // csrc/marching_cubes/dual_mc_inds.cu:45-182, dual_mc.cu:20-189).
 #include <algorithm>
+#include <climits>
 #include "ngs_common.cuh"
 #include "hash_table.cuh"
 
@@ -53,12 +54,13 @@ NGS_DEV float sdf_interp(const float* p1, const float* p2, float v1, float v2, f
 // (dual_mc_inds.cu:86,115,135): such a cube's count ends above 8 and the cube is dropped by
 // ngs_dual_mc_select, which keeps the cubes with exactly 8 writes; every probe therefore writes its
 // slots unconditionally and adds to the count without reading it back.
+// faces = 0: corner and edge probes only (the faces are taken by dual_faces_kernel).
 template <typename Lookup, typename Idx, int W>
 __global__ void dual_inds_kernel(Lookup lk, const int32_t* __restrict__ pb, Idx n_primal, int stride, int depth,
-                                 int64_t idx_base, int32_t* __restrict__ acc, int32_t* __restrict__ cnt) {
+                                 int64_t idx_base, int32_t* __restrict__ acc, int32_t* __restrict__ cnt, int faces) {
   const Idx sm1 = (Idx)stride - 1;
   const Idx n_corner = n_primal * 8, n_edge = n_primal * 12 * sm1;
-  const Idx total = n_corner + n_edge + n_primal * 6 * sm1 * sm1;
+  const Idx total = n_corner + n_edge + (faces ? n_primal * 6 * sm1 * sm1 : 0);
   for (Idx t = (Idx)ngs_gtid(); t < total; t += (Idx)ngs_gstride()) {
     Idx pid;
     // the probe's offset from the cell's base corner and its slots, kept in registers (axes are
@@ -140,32 +142,243 @@ __global__ void dual_inds_kernel(Lookup lk, const int32_t* __restrict__ pb, Idx 
 // Probes of n_primal cells of stride s: launch over 32-bit indices when they fit.
 template <typename Lookup, int W>
 void launch_dual_inds_w(Lookup lk, const int32_t* pb, int64_t n_primal, int stride, int depth, int64_t idx_base,
-                        int32_t* acc, int32_t* cnt, cudaStream_t s) {
-  const int64_t per = 8 + 12 * (int64_t)(stride - 1) + 6 * (int64_t)(stride - 1) * (stride - 1);
+                        int32_t* acc, int32_t* cnt, int faces, cudaStream_t s) {
+  const int64_t per = 8 + 12 * (int64_t)(stride - 1) + (faces ? 6 * (int64_t)(stride - 1) * (stride - 1) : 0);
   const int64_t total = n_primal * per;
   const unsigned grid = ngs_blocks(total, 256);
   ngs_count_launch();
   // 32-bit indexing needs the whole index space plus one grid stride below 2^32
   if (total + (int64_t)grid * 256 < (int64_t)UINT32_MAX)
     dual_inds_kernel<Lookup, uint32_t, W><<<grid, 256, 0, s>>>(lk, pb, (uint32_t)n_primal, stride, depth, idx_base, acc,
-                                                               cnt);
+                                                               cnt, faces);
   else
-    dual_inds_kernel<Lookup, int64_t, W><<<grid, 256, 0, s>>>(lk, pb, n_primal, stride, depth, idx_base, acc, cnt);
+    dual_inds_kernel<Lookup, int64_t, W><<<grid, 256, 0, s>>>(lk, pb, n_primal, stride, depth, idx_base, acc, cnt,
+                                                              faces);
 }
 
 // slot_words 2: the reference's (primal id, depth) pairs; 1: primal ids alone (the dual MC passes
 // read nothing else)
 template <typename Lookup>
 void launch_dual_inds(Lookup lk, const int32_t* pb, int64_t n_primal, int stride, int depth, int64_t idx_base,
-                      int32_t* acc, int slot_words, int32_t* cnt, cudaStream_t s) {
-  if (slot_words == 2) launch_dual_inds_w<Lookup, 2>(lk, pb, n_primal, stride, depth, idx_base, acc, cnt, s);
-  else launch_dual_inds_w<Lookup, 1>(lk, pb, n_primal, stride, depth, idx_base, acc, cnt, s);
+                      int32_t* acc, int slot_words, int32_t* cnt, cudaStream_t s, int faces = 1) {
+  if (slot_words == 2) launch_dual_inds_w<Lookup, 2>(lk, pb, n_primal, stride, depth, idx_base, acc, cnt, faces, s);
+  else launch_dual_inds_w<Lookup, 1>(lk, pb, n_primal, stride, depth, idx_base, acc, cnt, faces, s);
 }
 
 struct GridLookup {
   ngs_grid g;
   NGS_DEV int64_t operator()(int x, int y, int z) const { return grid_row(g, x, y, z); }
+  template <int K>
+  NGS_DEV void zrun(int x, int y, int z, int32_t (&r)[K]) const { grid_rows_zrun<K>(g, x, y, z, r); }
 };
+
+// Two-level rank bitmap (ngs_grid2): the outer grid has a bit per 64-cell word along z, and only the words
+// that hold a cell exist, in the order of the outer grid's ranks -- rows are ranks in (x, y, z) order, as
+// in the plain grid.  A lookup is two dependent 16-byte loads.
+struct Grid2Lookup {
+  ngs_grid2 g;
+  // the inner word of cells (x, y, 64 zw ..) relative to the box, or -1
+  NGS_DEV int64_t word(int x, int y, int zw) const {
+    const ngs_grid& o = g.outer;
+    const int i = x - o.origin[0], j = y - o.origin[1];
+    if ((i | j | zw) < 0 || i >= o.dims[0] || j >= o.dims[1] || zw >= o.dims[2]) return -1;
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(o.words) + ((int64_t)i * o.dims[1] + j) * o.zwords + (zw >> 6));
+    const unsigned long long bits = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+    const int b = zw & 63;
+    if (!((bits >> b) & 1ull)) return -1;
+    return (int64_t)v.x + __popcll(bits & ((1ull << b) - 1ull));
+  }
+  NGS_DEV int64_t operator()(int x, int y, int z) const {
+    int32_t r[1];
+    zrun<1>(x, y, z, r);
+    return r[0];
+  }
+  template <int K>
+  NGS_DEV void zrun(int x, int y, int z, int32_t (&r)[K]) const {
+    const int k0 = z - g.outer.origin[2];
+    int have = INT32_MIN;
+    uint4 v = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int t = 0; t < K; t++) {
+      const int k = k0 + t, zw = k >> 6;
+      if (zw != have) {
+        const int64_t w = word(x, y, zw);
+        v = w >= 0 ? __ldg(reinterpret_cast<const uint4*>(g.inner) + w) : make_uint4(0, 0, 0, 0);
+        have = zw;
+      }
+      const unsigned long long bits = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+      const int b = k & 63;
+      r[t] = (bits >> b) & 1ull ? (int32_t)(v.x + (unsigned)__popcll(bits & ((1ull << b) - 1ull))) : -1;
+    }
+  }
+};
+
+// Occupancy of 32 x 32 columns x one word of the box, a bit each: index of the block of (x, y, zw).
+NGS_DEV int64_t grid2_block(const ngs_grid& o, int x, int y, int zw) {
+  const int nby = ((o.origin[1] + o.dims[1] - 1) >> 5) - (o.origin[1] >> 5) + 1;
+  return ((int64_t)((x >> 5) - (o.origin[0] >> 5)) * nby + ((y >> 5) - (o.origin[1] >> 5))) * o.dims[2] + zw;
+}
+
+static int64_t grid2_blocks(const ngs_grid& o) {
+  const int64_t nbx = ((o.origin[0] + o.dims[0] - 1) >> 5) - (o.origin[0] >> 5) + 1;
+  const int64_t nby = ((o.origin[1] + o.dims[1] - 1) >> 5) - (o.origin[1] >> 5) + 1;
+  return nbx * nby * o.dims[2];
+}
+
+extern "C" size_t ngs_grid2_block_bytes(ngs_grid outer) {
+  return outer.dims[0] < 1 || outer.dims[1] < 1 || outer.dims[2] < 1 ? 0 : (size_t)((grid2_blocks(outer) + 31) / 32 * 4);
+}
+
+// Marks a cell: in the outer grid and the block bits (pass 0), or its bit in its inner word (pass 1).
+template <int PASS>
+NGS_DEV void grid2_mark(const Grid2Lookup& lk, int x, int y, int z) {
+  const ngs_grid& o = lk.g.outer;
+  const int k = z - o.origin[2], zw = k >> 6;
+  if constexpr (PASS == 0) {
+    const int i = x - o.origin[0], j = y - o.origin[1];
+    if ((i | j | k) < 0 || i >= o.dims[0] || j >= o.dims[1] || zw >= o.dims[2]) return;
+    unsigned long long* bits = &(static_cast<GridWord*>(o.words) + ((int64_t)i * o.dims[1] + j) * o.zwords + (zw >> 6))->bits;
+    const unsigned long long m = 1ull << (zw & 63);
+    if (*reinterpret_cast<volatile unsigned long long*>(bits) & m) return;
+    atomicOr(bits, m);
+    const int64_t b = grid2_block(o, x, y, zw);
+    if (!(*reinterpret_cast<volatile unsigned*>(lk.g.blocks + (b >> 5)) & (1u << (b & 31))))
+      atomicOr(lk.g.blocks + (b >> 5), 1u << (b & 31));
+  } else {
+    const int64_t w = lk.word(x, y, zw);
+    if (w < 0) return;
+    unsigned long long* bits = &(static_cast<GridWord*>(lk.g.inner) + w)->bits;
+    const unsigned long long m = 1ull << (k & 63);
+    if (!(*reinterpret_cast<volatile unsigned long long*>(bits) & m)) atomicOr(bits, m);
+  }
+}
+
+// The 27 sample corners c * 2 + {0, s, 2s}^3 of leaf cells (as ngs_grid_mark_cell_corners), a thread per
+// (cell, x, y) column.
+template <int PASS>
+__global__ void grid2_mark_cells_kernel(Grid2Lookup lk, const int32_t* __restrict__ c, int64_t n, int s) {
+  const int64_t total = n * 9;
+  for (int64_t t = ngs_gtid(); t < total; t += ngs_gstride()) {
+    const int64_t i = t / 9;
+    const int col = (int)(t - i * 9);
+    const int x = c[i * 3] * 2 + (col / 3) * s, y = c[i * 3 + 1] * 2 + (col % 3) * s, z = c[i * 3 + 2] * 2;
+#pragma unroll
+    for (int k = 0; k < 3; k++) grid2_mark<PASS>(lk, x, y, z + k * s);
+  }
+}
+
+// coords[i] + offsets[j] * scale (as ngs_grid_mark_coords).
+template <int PASS>
+__global__ void grid2_mark_coords_kernel(Grid2Lookup lk, const int32_t* __restrict__ c, int64_t n,
+                                         const int32_t* __restrict__ off, int n_off, int scale) {
+  const int64_t total = n * n_off;
+  for (int64_t t = ngs_gtid(); t < total; t += ngs_gstride()) {
+    const int64_t i = t / n_off;
+    const int o = (int)(t - i * n_off);
+    grid2_mark<PASS>(lk, c[i * 3] + off[o * 3] * scale, c[i * 3 + 1] + off[o * 3 + 1] * scale,
+                     c[i * 3 + 2] + off[o * 3 + 2] * scale);
+  }
+}
+
+static bool grid2_ok(const ngs_grid2& g, int pass) {
+  const ngs_grid& o = g.outer;
+  return o.words && o.stride == 1 && o.dims[0] > 0 && o.dims[1] > 0 && o.dims[2] > 0 &&
+         o.zwords == (o.dims[2] + 63) / 64 && (pass == 0 ? g.blocks != nullptr : g.inner != nullptr) &&
+         ((reinterpret_cast<uintptr_t>(o.words) | reinterpret_cast<uintptr_t>(g.inner)) & 15u) == 0;
+}
+
+extern "C" int ngs_grid2_mark_cell_corners(ngs_grid2 g, int pass, const int32_t* cells, int64_t n, int stride,
+                                           ngs_stream s) {
+  if (!grid2_ok(g, pass) || (pass != 0 && pass != 1) || n < 0 || stride < 1 || (n > 0 && !cells)) return NGS_ERR_INVALID_ARG;
+  if (n == 0) return NGS_OK;
+  ngs_count_launch();
+  if (pass == 0) grid2_mark_cells_kernel<0><<<ngs_blocks(n * 9, 256), 256, 0, (cudaStream_t)s>>>({g}, cells, n, stride);
+  else grid2_mark_cells_kernel<1><<<ngs_blocks(n * 9, 256), 256, 0, (cudaStream_t)s>>>({g}, cells, n, stride);
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}
+
+extern "C" int ngs_grid2_mark_coords(ngs_grid2 g, int pass, const int32_t* coords, int64_t n, const int32_t* offsets,
+                                     int n_off, int offset_scale, ngs_stream s) {
+  if (!grid2_ok(g, pass) || (pass != 0 && pass != 1) || n < 0 || n_off < 0 || (n > 0 && n_off > 0 && (!coords || !offsets)))
+    return NGS_ERR_INVALID_ARG;
+  if (n == 0 || n_off == 0) return NGS_OK;
+  const unsigned grid = ngs_blocks(n * n_off, 256);
+  ngs_count_launch();
+  if (pass == 0) grid2_mark_coords_kernel<0><<<grid, 256, 0, (cudaStream_t)s>>>({g}, coords, n, offsets, n_off, offset_scale);
+  else grid2_mark_coords_kernel<1><<<grid, 256, 0, (cudaStream_t)s>>>({g}, coords, n, offsets, n_off, offset_scale);
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}
+
+// The interior points of the six faces of primal cells of stride s >= 32, four slots each, found from the
+// dual centres that exist instead of by probing (s - 1)^2 points a face: a warp per 32-point strip of a
+// face and z word (faces along z: a lane reads the one word of its column) or per 32 x 32 points (faces
+// across z), skipped at once where the block has no centre at all.  Cell bases are multiples of s, so
+// the strips and tiles lie within one block.
+template <int W>
+__global__ void __launch_bounds__(256) dual_faces_kernel(Grid2Lookup lk, const int32_t* __restrict__ pb, int64_t n_primal,
+                                                         int s, int depth, int64_t idx_base, int32_t* __restrict__ acc,
+                                                         int32_t* __restrict__ cnt) {
+  const ngs_grid& o = lk.g.outer;
+  const int lane = threadIdx.x & 31;
+  const int tiles = s / 32, nz = max(s / 64, 1) + 1;
+  const int along = 4 * tiles * nz, units = along + 2 * tiles * tiles;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  auto occupied = [&](int x, int y, int zw) {
+    const int i = x - o.origin[0], j = y - o.origin[1];
+    // the block may reach past the box on either side; its bits exist if any of its columns does
+    if (zw < 0 || zw >= o.dims[2] || i + 31 < 0 || j + 31 < 0 || i >= o.dims[0] || j >= o.dims[1]) return false;
+    const int64_t b = grid2_block(o, max(x, o.origin[0]), max(y, o.origin[1]), zw);
+    return ((__ldg(lk.g.blocks + (b >> 5)) >> (b & 31)) & 1u) != 0u;
+  };
+  for (int64_t t = ngs_gtid() >> 5; t < n_primal * units; t += warps) {       // warp-uniform
+    const int64_t pid = t / units;
+    const int u = (int)(t - pid * units);
+    const int b[3] = {pb[pid * 3], pb[pid * 3 + 1], pb[pid * 3 + 2]};
+    const int32_t id = (int32_t)(pid + idx_base);
+    auto put = [&](int64_t row, int ax, int side) {
+      atomicAdd(cnt + row, 4);
+      const int b0 = ax == 0 ? 1 : 0, b1 = ax == 2 ? 1 : 2;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int slot = c_octant_slot[((1 - side) << ax) + ((k & 1) << b0) + ((k >> 1) << b1)];
+        if constexpr (W == 2) reinterpret_cast<int2*>(acc)[row * 8 + slot] = make_int2(id, depth);
+        else acc[row * 8 + slot] = id;
+      }
+    };
+    if (u < along) {
+      const int f = u / (tiles * nz), rem = u - f * tiles * nz, tile = rem / nz;
+      const int ax = f >> 1, side = f & 1;
+      const int zw = ((b[2] + 1 - o.origin[2]) >> 6) + rem - tile * nz;
+      const int z0 = zw * 64, lo = max(b[2] + 1 - o.origin[2], z0) - z0, hi = min(b[2] + s - 1 - o.origin[2], z0 + 63) - z0;
+      const int fixed = b[ax] + side * s, first = b[1 - ax] + tile * 32;
+      if (lo > hi || !occupied(ax == 0 ? fixed : first, ax == 0 ? first : fixed, zw)) continue;
+      if (tile == 0 && lane == 0) continue;                                    // the edge of the face
+      const int64_t w = lk.word(ax == 0 ? fixed : first + lane, ax == 0 ? first + lane : fixed, zw);
+      if (w < 0) continue;
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(lk.g.inner) + w);
+      const unsigned long long bits = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+      unsigned long long left = bits & (~0ull << lo) & (~0ull >> (63 - hi));
+      while (left) {
+        const int k = __ffsll((long long)left) - 1;
+        left &= left - 1ull;
+        put((int64_t)v.x + __popcll(bits & ((1ull << k) - 1ull)), ax, side);
+      }
+    } else {
+      const int v = u - along, side = v / (tiles * tiles), tt = v - side * tiles * tiles;
+      const int tx = tt / tiles, ty = tt - tx * tiles;
+      const int x0 = b[0] + tx * 32, y = b[1] + ty * 32 + lane, z = b[2] + side * s;
+      if (!occupied(x0, b[1] + ty * 32, (z - o.origin[2]) >> 6)) continue;
+      if (ty == 0 && lane == 0) continue;
+      for (int x = tx == 0 ? 1 : 0; x < 32; x++) {
+        const int64_t row = lk(x0 + x, y, z);
+        if (row >= 0) put(row, 2, side);
+      }
+    }
+  }
+}
+
 struct KeyLookup {
   const Slot* slots;
   int64_t mask;
@@ -184,8 +397,8 @@ struct KeyLookup {
 // along z) and takes one count update for all the samples that touch it; sample e reaches point p
 // through its corner q = p - e, which fills the slot of the octant opposite q -- the same slots and
 // counts as the per-sample probes of dual_inds_kernel.
-template <int W>
-__global__ void dual_inds_cells_kernel(ngs_grid dual, const int32_t* __restrict__ cells, int64_t n, int depth,
+template <typename Lookup, int W>
+__global__ void dual_inds_cells_kernel(Lookup dual, const int32_t* __restrict__ cells, int64_t n, int depth,
                                        int64_t idx_base, int32_t* __restrict__ acc, int32_t* __restrict__ cnt) {
   for (int64_t i = ngs_gtid(); i < n; i += ngs_gstride()) {
     const int x0 = cells[i * 3] * 2, y0 = cells[i * 3 + 1] * 2, z0 = cells[i * 3 + 2] * 2;
@@ -193,7 +406,7 @@ __global__ void dual_inds_cells_kernel(ngs_grid dual, const int32_t* __restrict_
     // the 9 runs looked up first, all their bitmap loads in flight together, then the updates
     int32_t r[9][3];
 #pragma unroll
-    for (int pxy = 0; pxy < 9; pxy++) grid_rows_zrun<3>(dual, x0 + pxy / 3, y0 + pxy % 3, z0, r[pxy]);
+    for (int pxy = 0; pxy < 9; pxy++) dual.template zrun<3>(x0 + pxy / 3, y0 + pxy % 3, z0, r[pxy]);
 #pragma unroll
     for (int pxy = 0; pxy < 9; pxy++) {
       const int px = pxy / 3, py = pxy % 3;
@@ -217,19 +430,55 @@ __global__ void dual_inds_cells_kernel(ngs_grid dual, const int32_t* __restrict_
   }
 }
 
-extern "C" int ngs_dual_mc_indices_cells(ngs_grid dual, const int32_t* cells, int64_t n_cells, int depth,
-                                         int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s) {
-  if (!dual.words || dual.stride != 1 || n_cells < 0 || (n_cells > 0 && (!cells || !acc || !cnt)))
-    return NGS_ERR_INVALID_ARG;
+template <typename Lookup>
+static int dual_inds_cells(Lookup lk, const int32_t* cells, int64_t n_cells, int depth, int64_t idx_base, int32_t* acc,
+                           int slot_words, int32_t* cnt, cudaStream_t s) {
+  if (n_cells < 0 || (n_cells > 0 && (!cells || !acc || !cnt))) return NGS_ERR_INVALID_ARG;
   if ((slot_words != 1 && slot_words != 2) || (reinterpret_cast<uintptr_t>(acc) & 7u)) return NGS_ERR_INVALID_ARG;
   if (n_cells == 0) return NGS_OK;
+  const unsigned grid = ngs_blocks(n_cells, 128);
   ngs_count_launch();
   if (slot_words == 2)
-    dual_inds_cells_kernel<2><<<ngs_blocks(n_cells, 128), 128, 0, (cudaStream_t)s>>>(dual, cells, n_cells, depth,
-                                                                                     idx_base, acc, cnt);
+    dual_inds_cells_kernel<Lookup, 2><<<grid, 128, 0, s>>>(lk, cells, n_cells, depth, idx_base, acc, cnt);
   else
-    dual_inds_cells_kernel<1><<<ngs_blocks(n_cells, 128), 128, 0, (cudaStream_t)s>>>(dual, cells, n_cells, depth,
-                                                                                     idx_base, acc, cnt);
+    dual_inds_cells_kernel<Lookup, 1><<<grid, 128, 0, s>>>(lk, cells, n_cells, depth, idx_base, acc, cnt);
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}
+
+extern "C" int ngs_dual_mc_indices_cells(ngs_grid dual, const int32_t* cells, int64_t n_cells, int depth,
+                                         int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s) {
+  if (!dual.words || dual.stride != 1) return NGS_ERR_INVALID_ARG;
+  return dual_inds_cells(GridLookup{dual}, cells, n_cells, depth, idx_base, acc, slot_words, cnt, (cudaStream_t)s);
+}
+
+extern "C" int ngs_dual_mc_indices_cells2(ngs_grid2 dual, const int32_t* cells, int64_t n_cells, int depth,
+                                          int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt, ngs_stream s) {
+  if (!grid2_ok(dual, 1)) return NGS_ERR_INVALID_ARG;
+  return dual_inds_cells(Grid2Lookup{dual}, cells, n_cells, depth, idx_base, acc, slot_words, cnt, (cudaStream_t)s);
+}
+
+extern "C" int ngs_dual_mc_indices_grid2(ngs_grid2 dual, const int32_t* primal_base, int64_t n_primal, int stride,
+                                         int depth, int64_t idx_base, int32_t* acc, int slot_words, int32_t* cnt,
+                                         ngs_stream s) {
+  if (!grid2_ok(dual, 1) || stride < 1 || n_primal < 0 || (n_primal > 0 && (!primal_base || !acc || !cnt)))
+    return NGS_ERR_INVALID_ARG;
+  if ((slot_words != 1 && slot_words != 2) || (reinterpret_cast<uintptr_t>(acc) & 7u)) return NGS_ERR_INVALID_ARG;
+  if (n_primal == 0) return NGS_OK;
+  // strides from 32 on: the faces from the centres that exist (a cell of the room's coarsest level would probe
+  // 6.3M points; all levels from 32 on together: under 2 ms, the probes 90)
+  const bool faces = stride >= 32 && dual.blocks;
+  launch_dual_inds(Grid2Lookup{dual}, primal_base, n_primal, stride, depth, idx_base, acc, slot_words, cnt,
+                   (cudaStream_t)s, !faces);
+  if (faces) {
+    const int tiles = stride / 32, nz = (stride >= 64 ? stride / 64 : 1) + 1;
+    const unsigned grid = ngs_blocks(n_primal * (4 * tiles * nz + 2 * tiles * tiles) * 32, 256);
+    ngs_count_launch();
+    if (slot_words == 2)
+      dual_faces_kernel<2><<<grid, 256, 0, (cudaStream_t)s>>>({dual}, primal_base, n_primal, stride, depth, idx_base, acc, cnt);
+    else
+      dual_faces_kernel<1><<<grid, 256, 0, (cudaStream_t)s>>>({dual}, primal_base, n_primal, stride, depth, idx_base, acc, cnt);
+  }
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }

@@ -55,7 +55,12 @@ class PcgConfig(C.Structure):
                 ("replace_every", C.c_int), ("blocks", C.c_int), ("timeout_s", C.c_double)]
 
 
-G, H = Grid, C.POINTER(HashTable)
+class Grid2(C.Structure):
+    """ngs_grid2: a two-level rank bitmap (the words of a box that hold a cell)."""
+    _fields_ = [("outer", Grid), ("inner", vp), ("blocks", vp)]
+
+
+G, H, G2 = Grid, C.POINTER(HashTable), Grid2
 PCG_BATCH_MAX = 64
 
 
@@ -160,6 +165,11 @@ _SIGS = {
     "ngs_primal_mc_count": ([vp, i64, C.c_int, vp, vp], C.c_int),
     "ngs_primal_mc_emit": ([vp, vp, i64, C.c_int, vp, vp, vp, vp, vp, vp], C.c_int),
     "ngs_dual_mc_indices_cells": ([G, vp, i64, C.c_int, i64, vp, C.c_int, vp, vp], C.c_int),
+    "ngs_grid2_block_bytes": ([G], sz),
+    "ngs_grid2_mark_cell_corners": ([G2, C.c_int, vp, i64, C.c_int, vp], C.c_int),
+    "ngs_grid2_mark_coords": ([G2, C.c_int, vp, i64, vp, C.c_int, C.c_int, vp], C.c_int),
+    "ngs_dual_mc_indices_grid2": ([G2, vp, i64, C.c_int, C.c_int, i64, vp, C.c_int, vp, vp], C.c_int),
+    "ngs_dual_mc_indices_cells2": ([G2, vp, i64, C.c_int, i64, vp, C.c_int, vp, vp], C.c_int),
     "ngs_grid_mark_cell_corners": ([G, vp, i64, C.c_int, vp], C.c_int),
     "ngs_dual_mc_indices_grid": ([G, vp, i64, C.c_int, C.c_int, i64, vp, C.c_int, vp, vp], C.c_int),
     "ngs_dual_mc_indices_hash": ([H, vp, i64, C.c_int, C.c_int, i64, vp, C.c_int, vp, vp], C.c_int),
