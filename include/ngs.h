@@ -345,6 +345,14 @@ typedef struct ngs_pcg_system {
                                 window, each block stages its slice of the search vector there;
                                 otherwise the launch reserves no shared memory for it and the space
                                 stays with the L1 cache that the gathers hit */
+  const int64_t* pk_start;   /* optional (MIXED, FP64): the recurrence matrix in the packed form below,
+                                [groups + 1] first unit of every group, pk_start[groups] = pk_units;
+                                vals32, col_delta and band are then not read (NULL: the CSR) */
+  const void* pk_vals;       /* [pk_units * 32] float (MIXED) or double (FP64) */
+  const int32_t* pk_cols;    /* [ngs_pcg_pack_col_words(n, pk_units, pk_wide)] */
+  int64_t pk_units;
+  int32_t pk_wide;           /* 4-byte columns; 0: 2-byte deltas, for |column - row| <= 32,767 */
+  int32_t pk_pad_;
 } ngs_pcg_system;
 
 typedef struct ngs_pcg_config {
@@ -357,6 +365,17 @@ typedef struct ngs_pcg_config {
   double timeout_s;          /* bound of every device-side wait */
 } ngs_pcg_config;
 
+/* The packed form of a matrix: four consecutive rows to a group, the group's entries in units of 8 per row
+ * (32 values, 32 columns), padded to the group's longest row.  count: units of every group (int32
+ * [ngs_pcg_pack_groups(n)]), whose exclusive scan is `start` ([groups + 1], the total at the end); fill writes
+ * the values (mode MIXED: float, FP64: double) and columns from the CSR. */
+int64_t ngs_pcg_pack_groups(int64_t n);
+int64_t ngs_pcg_pack_col_words(int64_t n, int64_t units, int wide);
+int ngs_pcg_pack_count(const int64_t* rowptr, int64_t n, int32_t* units, ngs_stream s);
+int ngs_pcg_pack_fill(const int64_t* rowptr, const int32_t* cols, const double* vals64, int64_t n,
+                      const int64_t* start, int wide, int mode, void* pk_vals, int32_t* pk_cols, ngs_stream s);
+/* inv_diag[i] = 1 / vals64[diag_slot[i]] (ngs_finish_system without the FP32 copy of the values) */
+int ngs_csr_inv_diag(const double* vals64, const int64_t* diag_slot, int64_t n, float* inv_diag, ngs_stream s);
 /* col_delta[j] = cols[j] - row(j) for a CSR whose every |column - row| fits int16 (the caller
  * checks the bound; ref: no counterpart, the reference's SpMV reads int32 columns,
  * csrc/sparse_solve/solve_pcg.cu:67-73). */

@@ -674,3 +674,17 @@ extern "C" int ngs_finish_system(const double* vals64, int64_t nnz, const int64_
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }
+
+__global__ void inv_diag_kernel(const double* __restrict__ v64, const int64_t* __restrict__ diag_slot, int64_t n,
+                                float* __restrict__ inv_diag) {
+  for (int64_t i = ngs_gtid(); i < n; i += ngs_gstride()) inv_diag[i] = (float)(1.0 / v64[diag_slot[i]]);
+}
+
+extern "C" int ngs_csr_inv_diag(const double* vals64, const int64_t* diag_slot, int64_t n, float* inv_diag,
+                                ngs_stream s) {
+  if (n < 0 || (n > 0 && (!vals64 || !diag_slot || !inv_diag))) return NGS_ERR_INVALID_ARG;
+  if (n == 0) return NGS_OK;
+  { ngs_count_launch(); inv_diag_kernel<<<ngs_blocks(n, 256), 256, 0, (cudaStream_t)s>>>(vals64, diag_slot, n, inv_diag); }
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}

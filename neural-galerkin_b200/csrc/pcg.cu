@@ -39,13 +39,16 @@
 // the solo one.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include "mf.cuh"
 
 constexpr int PCG_THREADS = 512;
 constexpr int PCG_MIN_BLOCKS = 2;      // blocks per SM the register budget is sized for
 constexpr int PCG_ROW_LANES = 8;       // lanes per row in the SpMV
+constexpr int PCG_GROUP_ROWS = 4;      // rows of a group of the packed form: a warp's, eight lanes each
 constexpr int PCG_ROW_COST = 8;        // work of a row on top of its non-zeros (vector traffic)
 constexpr int PCG_BLOCK_WORK = 16384;  // work (non-zeros + row cost) that justifies one more block
+constexpr double PCG_DRIFT = 16.0;     // true over recurrence residual (squared) that restarts the directions
 constexpr int PCG_CLUSTER_MAX = 16;    // CTAs of the largest thread-block cluster a small system gets
 constexpr int PCG_CLUSTER_NEED = 64;   // systems of at most this many blocks' work are solved by a cluster
 // Most blocks one cooperative solve may use (B200: 148 SMs x 2 = 296).  The capacity query clamps to
@@ -88,6 +91,10 @@ struct PcgArgs {
   int mf;                         // the matrix-free operator below replaces the CSR
   ngs_pcg_operator op;
   int win_cap;                    // elements of the search vector a block can stage in shared memory
+  const int64_t* pk_start;        // packed recurrence matrix (ngs_pcg_pack_*), or NULL
+  const void* pk_vals;
+  const void* pk_cols;
+  int pk_wide;                    // 4-byte columns instead of 2-byte deltas
 };
 
 // Shared memory (dynamic) of every PCG block for its window of the search vector: the SpMV of a
@@ -128,7 +135,16 @@ NGS_DEV bool block_rows(const PcgArgs& a, unsigned bid, int64_t& row0, int64_t& 
     row1 = (a.n * ((int64_t)bid + 1)) / a.nblocks;
     return true;
   }
-  if (threadIdx.x == 0) {
+  if (a.pk_start && threadIdx.x == 0) {
+    // packed: whole groups of rows, balanced by their units
+    const int64_t B = a.nblocks, G = (a.n + PCG_GROUP_ROWS - 1) / PCG_GROUP_ROWS, units = a.pk_start[G];
+    bounds[0] = min(a.n, PCG_GROUP_ROWS * first_row_at(a.pk_start, G, (units * (int64_t)bid) / B));
+    bounds[1] = bid + 1 == a.nblocks
+                    ? a.n
+                    : min(a.n, PCG_GROUP_ROWS * first_row_at(a.pk_start, G, (units * ((int64_t)bid + 1)) / B));
+    bad = 0;
+  }
+  if (!a.pk_start && threadIdx.x == 0) {
     const int64_t B = a.nblocks;
     bounds[0] = first_row_at(a.rowptr, a.n, (a.nnz * (int64_t)bid) / B);
     bounds[1] = bid + 1 == a.nblocks ? a.n : first_row_at(a.rowptr, a.n, (a.nnz * ((int64_t)bid + 1)) / B);
@@ -259,6 +275,104 @@ NGS_DEV void spmv_rows_plain(const PcgArgs& a, const MT* __restrict__ vals, cons
   }
   __syncthreads();
 }
+// Packed form: four consecutive rows to a group, eight lanes to a row, the group's entries in units of 8 per
+// row -- entry 8 k + l of a row is lane l's of unit k -- padded to the longest of the four rows (padding: the
+// row's own column, value 0).  A unit is 32 values and 32 columns side by side, so that a warp reads it with one
+// wavefront each, where four CSR rows that start anywhere take two to four; nothing is predicated and no row
+// pointer is read.  Columns are 2-byte deltas of two units in a word (group g's words start at unit
+// (start + g + 1) / 2 rounded down), or 4 bytes where the deltas do not fit.  The sums run over the
+// entries as in the row-at-a-time form.
+//
+// Bound: latency and wavefronts of the vector's gathers (a product of the 300k-point scene's level 0 gathers
+// 74M floats, half of them from L1; DRAM runs at 3.5 of 6.5 TB/s).  So up to 16 units (12 with 4-byte columns
+// or FP64 values, whose registers would spill) are loaded together and then gathered together, and the next
+// group's lines are prefetched to L2, which holds no register.  Measured, all solves of a level, CSR form ->
+// packed: 300k points 9.19 -> 8.30 and 3.53 -> 3.17 ms, 0.93 -> 0.76, 0.42 -> 0.43; 5M-point room 90.9 -> 73.3
+// and 15.9 -> 13.5 against the packed form without the prefetch.
+template <bool STREAM, bool WIDE, typename MT, typename VT, typename ACC, typename Pre, typename Epi>
+NGS_DEV void spmv_packed(const PcgArgs& a, const VT* v, int64_t row0, int64_t row1, Pre pre, Epi epi, double& dsum) {
+  constexpr int WARPS = PCG_THREADS / 32;
+  const int lane = threadIdx.x & 31, quarter = lane / PCG_ROW_LANES;
+  const MT* vals = static_cast<const MT*>(a.pk_vals) + lane;
+  const int32_t* cols = static_cast<const int32_t*>(a.pk_cols) + lane;
+  const int end = (int)((row1 + PCG_GROUP_ROWS - 1) / PCG_GROUP_ROWS);
+  int g = (int)(row0 / PCG_GROUP_ROWS) + (threadIdx.x >> 5);
+  // first unit, and the one past the last, of this group and of the next
+  int first = 0, past = 0, next = 0, after = 0;
+  auto range = [&](int q, int& lo, int& hi) {
+    if (q >= end) {
+      lo = hi = 0;
+      return;
+    }
+    lo = (int)a.pk_start[q];
+    hi = (int)a.pk_start[q + 1];
+  };
+  range(g, first, past);
+  range(g + WARPS, next, after);
+  for (; g < end; g += WARPS) {                                     // warp-uniform
+    const int n = past - first;
+    // the next group's lines on their way to L2 (no registers held): a line per lane
+    {
+      constexpr int LINES = sizeof(MT) / 4;                         // of a unit's values
+      const char* nv = static_cast<const char*>(a.pk_vals) + (int64_t)next * 32 * sizeof(MT);
+      const char* nc = static_cast<const char*>(a.pk_cols) +
+                       (int64_t)(WIDE ? next : ((next + g + WARPS + 1) >> 1)) * 128;
+      const int lv = (after - next) * LINES, lc = WIDE ? after - next : (after - next + 1) / 2;
+      for (int l = lane; l < lv + lc; l += 32)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(l < lv ? nv + l * 128 : nc + (l - lv) * 128));
+    }
+    int next2, after2;
+    range(g + 2 * WARPS, next2, after2);
+    const int row = g * PCG_GROUP_ROWS + quarter, own = min(row, (int)a.n - 1);
+    const bool writes = (lane & (PCG_ROW_LANES - 1)) == 0 && row < (int)row1;
+    double2 ax = make_double2(0.0, 0.0);
+    if (writes) ax = pre(row);
+    ACC acc = (ACC)0;
+    // up to UB units at once: their loads in flight together, then their gathers; rounds of eight summed in MT
+    auto batch = [&](auto ub, int k0) {
+      constexpr int UB = decltype(ub)::value, CW = WIDE ? UB : UB / 2;
+      const MT* mv = vals + (int64_t)(first + k0) * 32;
+      const int32_t* cv = cols + (int64_t)(WIDE ? first + k0 : ((first + g + 1) >> 1) + k0 / 2) * 32;
+      const int left = n - k0;
+      MT m[UB];
+      int32_t c[CW];
+      VT x[UB];
+#pragma unroll
+      for (int k = 0; k < CW; k++) c[k] = (WIDE ? k : 2 * k) < left ? ld_mat<STREAM>(cv + k * 32) : (WIDE ? own : 0);
+#pragma unroll
+      for (int k = 0; k < UB; k++) m[k] = k < left ? ld_mat<STREAM>(mv + k * 32) : (MT)0;
+#pragma unroll
+      for (int k = 0; k < UB; k++) {
+        if constexpr (WIDE) x[k] = v[c[k]];
+        else x[k] = v[own + ((k & 1) ? c[k / 2] >> 16 : (int32_t)(int16_t)c[k / 2])];
+      }
+#pragma unroll
+      for (int k8 = 0; k8 < UB; k8 += 8) {
+        MT r0 = (MT)0, r1 = (MT)0;
+#pragma unroll
+        for (int k = k8; k < k8 + 8 && k < UB; k += 2) {
+          r0 += m[k] * (MT)x[k];
+          r1 += m[k + 1] * (MT)x[k + 1];
+        }
+        acc += (ACC)r0 + (ACC)r1;
+      }
+    };
+    constexpr int MOST = sizeof(MT) == 8 || WIDE ? 8 : 16;           // rounds of eight either way: the same sums
+    int k0 = 0;
+    for (; n - k0 > 12; k0 += MOST) batch(std::integral_constant<int, MOST>{}, k0);
+    if (n - k0 > 8) batch(std::integral_constant<int, 12>{}, k0);
+    else if (n - k0 > 0) batch(std::integral_constant<int, 8>{}, k0);
+    first = next;
+    past = after;
+    next = next2;
+    after = after2;
+#pragma unroll
+    for (int o = PCG_ROW_LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (writes) dsum += epi(row, (double)acc, ax);
+  }
+  __syncthreads();
+}
+
 // The streaming choice is a template argument: one load form per instantiation (a runtime choice
 // per load cost 7 % of the level-0 solve and forced register spills).  FORM picks the SpMV form at
 // compile time (kernels specialised per form, so that one form's register allocation is not shaped
@@ -266,7 +380,7 @@ NGS_DEV void spmv_rows_plain(const PcgArgs& a, const MT* __restrict__ vals, cons
 // a batch or a cluster launch).  Each form runs the same uncontracted arithmetic in every kernel, so
 // a system's result does not depend on which kernel solved it.
 constexpr int PCG_FORM_ANY = 0, PCG_FORM_DELTA_STREAM = 1, PCG_FORM_DELTA = 2, PCG_FORM_COLS_STREAM = 3,
-              PCG_FORM_COLS = 4;
+              PCG_FORM_COLS = 4, PCG_FORM_PACKED = 5;      // 5 .. 8: + 1 streamed, + 2 4-byte columns
 
 template <int FORM, typename MT, typename VT, typename ACC, typename Pre, typename Epi>
 NGS_DEV void spmv_rows(const PcgArgs& a, const MT* __restrict__ vals, const VT* v, int64_t voff, int64_t row0,
@@ -277,7 +391,7 @@ NGS_DEV void spmv_rows(const PcgArgs& a, const MT* __restrict__ vals, const VT* 
     spmv_rows_piped<false, true, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
   } else if constexpr (FORM == PCG_FORM_COLS_STREAM) {
     spmv_rows_plain<true, false, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
-  } else if constexpr (FORM == PCG_FORM_COLS) {
+  } else if constexpr (FORM == PCG_FORM_COLS || FORM >= PCG_FORM_PACKED) {   // packed: the true residual's
     spmv_rows_plain<false, false, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
   } else if (a.cols16) {
     // the column encoding too: 2-byte deltas when the caller supplied them, 4-byte columns otherwise
@@ -286,6 +400,18 @@ NGS_DEV void spmv_rows(const PcgArgs& a, const MT* __restrict__ vals, const VT* 
   } else {
     if (a.evict_first) spmv_rows_plain<true, false, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
     else spmv_rows_plain<false, false, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
+  }
+}
+
+// The recurrence matrix of a packed system.
+template <typename MT, typename VT, typename ACC, typename Pre, typename Epi>
+NGS_DEV void spmv_packed_any(const PcgArgs& a, const VT* v, int64_t row0, int64_t row1, Pre pre, Epi epi, double& dsum) {
+  if (a.pk_wide) {
+    if (a.evict_first) spmv_packed<true, true, MT, VT, ACC>(a, v, row0, row1, pre, epi, dsum);
+    else spmv_packed<false, true, MT, VT, ACC>(a, v, row0, row1, pre, epi, dsum);
+  } else {
+    if (a.evict_first) spmv_packed<true, false, MT, VT, ACC>(a, v, row0, row1, pre, epi, dsum);
+    else spmv_packed<false, false, MT, VT, ACC>(a, v, row0, row1, pre, epi, dsum);
   }
 }
 
@@ -572,6 +698,16 @@ NGS_DEV void pcg_body(const PcgArgs& a, const unsigned bid, Sync& sy) {
     if (!a.mf && rows_ok && a.win_cap > 0) csr_window(a, row0, row1, win_bounds[0], win_bounds[1]);
   }
   auto spmv_w = [&](double& sum) {
+    if constexpr (FORM >= PCG_FORM_PACKED) {
+      constexpr int F = FORM - PCG_FORM_PACKED;
+      spmv_packed<(F & 1) != 0, (F & 2) != 0, MT, VT, ACC>(a, u, row0, row1, w_pre, w_epi, sum);
+      return;
+    } else if constexpr (FORM == PCG_FORM_ANY) {
+      if (a.pk_start) {
+        spmv_packed_any<MT, VT, ACC>(a, u, row0, row1, w_pre, w_epi, sum);
+        return;
+      }
+    }
     const int64_t wlo = (int64_t)win_bounds[0], wn = (int64_t)win_bounds[1] - wlo;
     if (wn > 0 && wn <= a.win_cap) {
       VT* win = reinterpret_cast<VT*>(pcg_win_raw);
@@ -710,28 +846,36 @@ NGS_DEV void pcg_body(const PcgArgs& a, const unsigned bid, Sync& sy) {
     if (!apply_w(part[1])) return pcg_abandon(a, it);
     if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
     it++;
-    const double gamma_new = res[0];
+    double gamma_new = res[0];
     delta = res[1];
     rho = res[2];
     if (sqrt(rho) <= target) {
       if (MODE != NGS_PCG_MIXED) { converged = true; break; }
-      // end of an inner solve: true FP64 residual, stop or restart the recurrences from it
+      // the recurrence residual is down: the true FP64 residual takes its place
       if (!sy.barrier()) return pcg_abandon(a, it);
       part[0] = part[1] = part[2] = 0.0;
       if (!apply_true(part[2])) return pcg_abandon(a, it);
       replacements++;
       for (int64_t i = i0; i < i1; i += is) part[0] += (double)r[i] * (double)u[i];
-      if (!sy.barrier()) return pcg_abandon(a, it);
-      if (!apply_w(part[1])) return pcg_abandon(a, it);
       if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
+      const double rec = rho;
+      gamma_new = res[0];
       rho = res[2];
       if (sqrt(rho) <= atol) { converged = true; break; }
-      gamma = res[0];
+      part[0] = part[1] = part[2] = 0.0;
+      if (!apply_w(part[1])) return pcg_abandon(a, it);
+      if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
       delta = res[1];
-      alpha = delta != 0.0 ? gamma / delta : 0.0;
-      beta = 0.0;
       target = fmax(atol, rtol_inner * sqrt(rho));
-      continue;
+      // The search directions go on from the replaced residual; only where the recurrence had drifted far from
+      // it do they start anew.  (Starting anew at every refinement lost the directions that the conjugate
+      // gradients had found: 54 iterations instead of 52 on level 0 of a 300k-point cloud.)
+      if (rho > PCG_DRIFT * rec) {
+        gamma = gamma_new;
+        alpha = delta != 0.0 ? gamma / delta : 0.0;
+        beta = 0.0;
+        continue;
+      }
     }
     beta = gamma != 0.0 ? gamma_new / gamma : 0.0;
     const double den = delta - beta * gamma_new / alpha;
@@ -851,6 +995,10 @@ static int pcg_capacity() {
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_DELTA>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_COLS_STREAM>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_COLS>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_PACKED>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_PACKED + 1>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_PACKED + 2>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_form_kernel<MODE, PCG_FORM_PACKED + 3>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_kernel<MODE, PCG_OPS_MF>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_MF>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_BOTH>));
@@ -916,6 +1064,7 @@ static int pcg_cluster_limit() {
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_kernel<MODE, PCG_OPS_MF>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_DELTA>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_COLS>));
+    limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED>));
   }
   if (limit > PCG_CLUSTER_MAX) limit = PCG_CLUSTER_MAX;
   if (dev >= 0 && dev < 64) cached[dev] = limit > 0 ? limit : -1;
@@ -982,7 +1131,12 @@ static void* pcg_cluster_kernel_of(int mode, bool mf) {
 // (level 1 of a 300k-point cloud: 3.51 against 3.76 ms with 4-byte columns); without it, the 4-byte
 // columns in the row-at-a-time loop when the caller supplied both (its level 0: 9.22 against 9.34
 // ms).  Solo and batched solves of a system take the same decision, so their results stay identical.
+// A packed system takes neither: its columns are in the packed form.
 static void pcg_set_window(PcgArgs& a, int mode, int64_t band, int64_t nblocks) {
+  if (a.pk_start) {
+    a.win_cap = 0;
+    return;
+  }
   const int64_t cap = PCG_WIN_BYTES / (int64_t)pcg_vec_bytes(mode);
   const int64_t rows = nblocks > 0 ? (a.n + nblocks - 1) / nblocks : a.n;
   a.win_cap = (!a.mf && band > 0 && rows + 2 * band <= cap) ? (int)cap : 0;
@@ -1014,7 +1168,10 @@ static int launch_cluster(PcgArgs& a, int mode, int csize, cudaStream_t st) {
   void* args[] = {&a};
   ngs_count_launch();
   const void* f = pcg_cluster_kernel_of(mode, a.mf != 0);
-  if (!a.mf && !a.evict_first && (mode == NGS_PCG_MIXED || mode == NGS_PCG_FP64)) {
+  if (!a.mf && a.pk_start && !a.pk_wide && !a.evict_first && (mode == NGS_PCG_MIXED || mode == NGS_PCG_FP64)) {
+    f = mode == NGS_PCG_MIXED ? (const void*)pcg_cluster_form_kernel<NGS_PCG_MIXED, PCG_FORM_PACKED>
+                              : (const void*)pcg_cluster_form_kernel<NGS_PCG_FP64, PCG_FORM_PACKED>;
+  } else if (!a.mf && !a.pk_start && !a.evict_first && (mode == NGS_PCG_MIXED || mode == NGS_PCG_FP64)) {
     if (mode == NGS_PCG_MIXED)
       f = a.cols16 ? (const void*)pcg_cluster_form_kernel<NGS_PCG_MIXED, PCG_FORM_DELTA>
                    : (const void*)pcg_cluster_form_kernel<NGS_PCG_MIXED, PCG_FORM_COLS>;
@@ -1053,7 +1210,8 @@ static int prepare_pcg(const ngs_pcg_system* sys, const ngs_pcg_config* cfg, voi
   } else {
     if (!sys->rowptr || (sys->nnz > 0 && !sys->cols && !sys->col_delta)) return NGS_ERR_INVALID_ARG;
     if (mode == NGS_PCG_REFERENCE && (!sys->vals32 || !sys->b32 || !sys->x32)) return NGS_ERR_INVALID_ARG;
-    if (mode == NGS_PCG_MIXED && (!sys->vals32 || !sys->vals64 || !sys->b64 || !sys->x64)) return NGS_ERR_INVALID_ARG;
+    if (mode == NGS_PCG_REFERENCE && sys->pk_start) return NGS_ERR_INVALID_ARG;
+    if (mode == NGS_PCG_MIXED && ((!sys->vals32 && !sys->pk_start) || !sys->vals64 || !sys->b64 || !sys->x64)) return NGS_ERR_INVALID_ARG;
     if (mode == NGS_PCG_FP64 && (!sys->vals64 || !sys->b64 || !sys->x64)) return NGS_ERR_INVALID_ARG;
   }
   if (!ws || ws_bytes < ngs_pcg_workspace_bytes(sys->n, mode)) return NGS_ERR_OOM;
@@ -1096,6 +1254,15 @@ static int prepare_pcg(const ngs_pcg_system* sys, const ngs_pcg_config* cfg, voi
   a.win_cap = 0;                       // decided with the block count (pcg_set_window)
   const size_t mat_bytes = (size_t)sys->nnz * ((sys->col_delta ? 2 : 4) + (mode == NGS_PCG_FP64 ? 8 : 4));
   a.evict_first = mat_bytes > (size_t)96 << 20;
+  if (!op && sys->pk_start) {
+    if (!sys->pk_vals || !sys->pk_cols || !sys->cols || sys->pk_units < 0) return NGS_ERR_INVALID_ARG;
+    a.pk_start = sys->pk_start;
+    a.pk_vals = sys->pk_vals;
+    a.pk_cols = sys->pk_cols;
+    a.pk_wide = sys->pk_wide;
+    a.cols16 = nullptr;
+    a.evict_first = (size_t)sys->pk_units * 32 * ((sys->pk_wide ? 4 : 2) + (mode == NGS_PCG_FP64 ? 8 : 4)) > (size_t)96 << 20;
+  }
   if (op) {
     a.mf = 1;
     a.op = *op;
@@ -1111,6 +1278,11 @@ static int prepare_pcg(const ngs_pcg_system* sys, const ngs_pcg_config* cfg, voi
 // for its SpMV form.
 template <int MODE>
 static void* pcg_form_kernel_for(const PcgArgs& a) {
+  if (a.pk_start) {
+    if (a.pk_wide)
+      return a.evict_first ? (void*)pcg_form_kernel<MODE, PCG_FORM_PACKED + 3> : (void*)pcg_form_kernel<MODE, PCG_FORM_PACKED + 2>;
+    return a.evict_first ? (void*)pcg_form_kernel<MODE, PCG_FORM_PACKED + 1> : (void*)pcg_form_kernel<MODE, PCG_FORM_PACKED>;
+  }
   if (a.cols16) return a.evict_first ? (void*)pcg_form_kernel<MODE, PCG_FORM_DELTA_STREAM> : (void*)pcg_form_kernel<MODE, PCG_FORM_DELTA>;
   return a.evict_first ? (void*)pcg_form_kernel<MODE, PCG_FORM_COLS_STREAM> : (void*)pcg_form_kernel<MODE, PCG_FORM_COLS>;
 }
@@ -1284,6 +1456,83 @@ extern "C" int ngs_pcg_solve_noalloc(const ngs_pcg_system* sys, const ngs_pcg_co
   // and the kernel initialises every vector and writes each partial before reading it, so what the
   // previous call left in the shared scratch does not matter.
   return ngs_pcg_solve(sys, cfg, ws, kNoallocScratchBytes, info_dev, resid_dev, s);
+}
+
+// ----------------------------------------------------------------------------- packed form
+__global__ void pack_count_kernel(const int64_t* __restrict__ rp, int64_t n, int64_t groups, int32_t* __restrict__ units) {
+  for (int64_t g = ngs_gtid(); g < groups; g += ngs_gstride()) {
+    int64_t most = 0;
+    for (int64_t r = g * PCG_GROUP_ROWS; r < min(n, (g + 1) * PCG_GROUP_ROWS); r++) most = max(most, rp[r + 1] - rp[r]);
+    units[g] = (int32_t)((most + PCG_ROW_LANES - 1) / PCG_ROW_LANES);
+  }
+}
+
+// A warp per group; the values come from the FP64 matrix.
+template <typename MT, bool WIDE>
+__global__ void pack_fill_kernel(const int64_t* __restrict__ rp, const int32_t* __restrict__ cols,
+                                 const double* __restrict__ vals, int64_t n, int64_t groups,
+                                 const int64_t* __restrict__ start, MT* __restrict__ out_vals,
+                                 int32_t* __restrict__ out_cols) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t g = ngs_gtid() >> 5; g < groups; g += warps) {
+    const int64_t row = g * PCG_GROUP_ROWS + lane / PCG_ROW_LANES, own = min(row, n - 1);
+    const int64_t e0 = row < n ? rp[row] : 0, e1 = row < n ? rp[row + 1] : 0;
+    const int64_t s0 = start[g];
+    const int units = (int)(start[g + 1] - s0);
+    int32_t low = 0;
+    for (int k = 0; k < units; k++) {
+      const int64_t e = e0 + k * PCG_ROW_LANES + (lane & (PCG_ROW_LANES - 1));
+      const bool in = e < e1;
+      out_vals[(s0 + k) * 32 + lane] = in ? (MT)vals[e] : (MT)0;
+      const int32_t col = in ? cols[e] : (int32_t)own;
+      if constexpr (WIDE) {
+        out_cols[(s0 + k) * 32 + lane] = col;
+      } else {
+        const int32_t d = (col - (int32_t)own) & 0xffff;
+        if (k & 1) out_cols[(((s0 + g + 1) >> 1) + k / 2) * 32 + lane] = low | (d << 16);
+        else low = d;
+      }
+    }
+    if (!WIDE && (units & 1)) out_cols[(((s0 + g + 1) >> 1) + units / 2) * 32 + lane] = low;
+  }
+}
+
+extern "C" int64_t ngs_pcg_pack_groups(int64_t n) { return n < 0 ? 0 : (n + PCG_GROUP_ROWS - 1) / PCG_GROUP_ROWS; }
+
+extern "C" int64_t ngs_pcg_pack_col_words(int64_t n, int64_t units, int wide) {
+  return (wide ? units : (units + ngs_pcg_pack_groups(n) + 2) / 2) * 32;
+}
+
+extern "C" int ngs_pcg_pack_count(const int64_t* rowptr, int64_t n, int32_t* units, ngs_stream s) {
+  if (n < 0 || (n > 0 && (!rowptr || !units))) return NGS_ERR_INVALID_ARG;
+  if (n == 0) return NGS_OK;
+  const int64_t groups = ngs_pcg_pack_groups(n);
+  { ngs_count_launch(); pack_count_kernel<<<ngs_blocks(groups, 256), 256, 0, (cudaStream_t)s>>>(rowptr, n, groups, units); }
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}
+
+extern "C" int ngs_pcg_pack_fill(const int64_t* rowptr, const int32_t* cols, const double* vals64, int64_t n,
+                                 const int64_t* start, int wide, int mode, void* pk_vals, int32_t* pk_cols,
+                                 ngs_stream s) {
+  if (n < 0 || (mode != NGS_PCG_MIXED && mode != NGS_PCG_FP64) ||
+      (n > 0 && (!rowptr || !cols || !vals64 || !start || !pk_vals || !pk_cols)))
+    return NGS_ERR_INVALID_ARG;
+  if (n == 0) return NGS_OK;
+  const int64_t groups = ngs_pcg_pack_groups(n);
+  const unsigned grid = ngs_blocks(groups * 32, 256);
+  cudaStream_t st = (cudaStream_t)s;
+  ngs_count_launch();
+  if (mode == NGS_PCG_MIXED) {
+    if (wide) pack_fill_kernel<float, true><<<grid, 256, 0, st>>>(rowptr, cols, vals64, n, groups, start, (float*)pk_vals, pk_cols);
+    else pack_fill_kernel<float, false><<<grid, 256, 0, st>>>(rowptr, cols, vals64, n, groups, start, (float*)pk_vals, pk_cols);
+  } else {
+    if (wide) pack_fill_kernel<double, true><<<grid, 256, 0, st>>>(rowptr, cols, vals64, n, groups, start, (double*)pk_vals, pk_cols);
+    else pack_fill_kernel<double, false><<<grid, 256, 0, st>>>(rowptr, cols, vals64, n, groups, start, (double*)pk_vals, pk_cols);
+  }
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
 }
 
 // ----------------------------------------------------------------------------- 2-byte column deltas

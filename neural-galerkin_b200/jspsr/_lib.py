@@ -47,7 +47,9 @@ class PcgOperator(C.Structure):
 class PcgSystem(C.Structure):
     _fields_ = [("n", C.c_int64), ("nnz", C.c_int64), ("rowptr", vp), ("cols", vp), ("vals32", vp),
                 ("vals64", vp), ("b32", vp), ("b64", vp), ("inv_diag", vp), ("x32", vp), ("x64", vp),
-                ("col_delta", vp), ("op", C.POINTER(PcgOperator)), ("band", C.c_int64)]
+                ("col_delta", vp), ("op", C.POINTER(PcgOperator)), ("band", C.c_int64), ("pk_start", vp),
+                ("pk_vals", vp), ("pk_cols", vp), ("pk_units", C.c_int64), ("pk_wide", C.c_int32),
+                ("pk_pad_", C.c_int32)]
 
 
 class PcgConfig(C.Structure):
@@ -125,6 +127,11 @@ _SIGS = {
     "ngs_correction_stiffness": ([vp, i64, C.c_int, G, vp, vp, vp, C.c_int, vp, vp], C.c_int),
     "ngs_correction_screen": ([vp, vp, i64, vp, vp, f64, vp, vp], C.c_int),
     "ngs_finish_system": ([vp, i64, vp, i64, vp, vp, vp], C.c_int),
+    "ngs_pcg_pack_groups": ([i64], i64),
+    "ngs_pcg_pack_col_words": ([i64, i64, C.c_int], i64),
+    "ngs_pcg_pack_count": ([vp, i64, vp, vp], C.c_int),
+    "ngs_pcg_pack_fill": ([vp, vp, vp, i64, vp, C.c_int, C.c_int, vp, vp, vp], C.c_int),
+    "ngs_csr_inv_diag": ([vp, vp, i64, vp, vp], C.c_int),
     "ngs_csr_col_delta": ([vp, vp, i64, vp, vp], C.c_int),
     "ngs_mf_count": ([vp, i64, i64, vp, vp, vp], C.c_int),
     "ngs_mf_fill": ([vp, vp, i64, vp, i64, vp, vp, vp, vp, vp, vp], C.c_int),

@@ -94,7 +94,7 @@ class Level:
     rowptr: torch.Tensor = None
     cols: torch.Tensor = None
     vals64: torch.Tensor = None
-    vals32: torch.Tensor = None
+    vals32_: torch.Tensor = None
     diag_slot: torch.Tensor = None
     inv_diag: torch.Tensor = None
     nnz: int = 0
@@ -106,9 +106,11 @@ class Level:
     x32: torch.Tensor = None
     info: torch.Tensor = None
     resid: torch.Tensor = None
-    col_delta: torch.Tensor = None   # int16 column - row per non-zero (when every delta fits)
-    delta_ok: bool = False
-    band: int = 0                    # bound on |column - row| (decides the solver's shared-memory window)
+    band: int = 0                    # bound on |column - row| (decides the packed form's column width)
+    pk_start: torch.Tensor = None    # the solver's packed copy of the matrix: first unit of every group of rows,
+    pk_units: int = 0                # units in all, values and columns
+    pk_vals: torch.Tensor = None
+    pk_cols: torch.Tensor = None
     # matrix-free operator (solver reads no CSR): the point basis transposed per row
     group: tuple = None            # (sorted cell keys, point order): screening terms of long-pair levels
     pair_form: bool = False        # screening terms gathered per row from the transposed pairs
@@ -119,6 +121,13 @@ class Level:
     n_pairs: int = 0                # E
     max_pairs: int = 0              # longest row list
     stencil: torch.Tensor = None    # [125] FP64 same-level stiffness
+
+    @property
+    def vals32(self):
+        """FP32 copy of the matrix values (the packed solver reads its own; made on request)."""
+        if self.vals32_ is None and self.vals64 is not None:
+            self.vals32_ = self.vals64.float()
+        return self.vals32_
 
 
 def _box(qmin, qmax, stride, pad=1):
@@ -485,6 +494,13 @@ class Reconstruction(DualMesher):
             L.call("ngs_stencil_count", lv.grid, L.ptr(lv.coords), lv.n, L.ptr(lv.masks), L.ptr(counts), st)
             lv.rowptr = torch.empty(lv.n + 1, dtype=torch.int64, device=self.dev)
             L.scan(counts, out=lv.rowptr[:lv.n], total=lv.rowptr[lv.n:])
+            if self.solver.mode in (L.PCG_MIXED, L.PCG_FP64):
+                # units of the solver's packed matrix per group of rows (its buffers are sized with the CSR's)
+                groups = L.load().ngs_pcg_pack_groups(lv.n)
+                units = torch.empty(groups, dtype=torch.int32, device=self.dev)
+                L.call("ngs_pcg_pack_count", L.ptr(lv.rowptr), lv.n, L.ptr(units), st)
+                lv.pk_start = torch.empty(groups + 1, dtype=torch.int64, device=self.dev)
+                L.scan(units, out=lv.pk_start[:groups], total=lv.pk_start[groups:])
             if self.alpha > 0 and (mf_candidate or self.pair_row_limit > 0):
                 # (point, slot) pairs per row (the screening terms in gather form; their counts also
                 # decide the matrix-free operator), the scan places the lists
@@ -493,18 +509,20 @@ class Reconstruction(DualMesher):
                 lv.t_ptr = torch.empty(lv.n + 1, dtype=torch.int64, device=self.dev)
                 L.scan(pc, out=lv.t_ptr[:lv.n], total=lv.t_ptr[lv.n:])
         self._mark("structure")
-        # with the non-zero counts, a bound on |column - row| per level (decides the 2-byte columns), and
-        # the pair counts (decide the matrix-free operator): one synchronisation for all levels
+        # with the non-zero counts, a bound on |column - row| per level (decides the 2-byte columns), the
+        # packed matrices' units and the pair counts (decide the matrix-free operator): one synchronisation for all levels
         span = [self._row_span_bound(lv) for lv in self.levels]
         pairs = [lv.t_ptr[lv.n] if lv.t_ptr is not None else torch.zeros((), dtype=torch.int64, device=self.dev)
                  for lv in self.levels]
-        host = torch.cat([torch.stack([lv.rowptr[lv.n] for lv in self.levels] + span + pairs),
+        units = [lv.pk_start[-1] if lv.pk_start is not None else lv.rowptr[lv.n] for lv in self.levels]
+        host = torch.cat([torch.stack([lv.rowptr[lv.n] for lv in self.levels] + span + pairs + units),
                           pair_max.long()]).cpu().numpy()
         D = self.depth
-        nnz, span, npairs, pmax = host[:D], host[D:2 * D], host[2 * D:3 * D], host[3 * D:]
+        nnz, span, npairs, units, pmax = host[:D], host[D:2 * D], host[2 * D:3 * D], host[3 * D:4 * D], host[4 * D:]
         for d, lv in enumerate(self.levels):
             lv.nnz = int(nnz[d])
             lv.band = int(span[d])
+            lv.pk_units = int(units[d])
             lv.n_pairs, lv.max_pairs = int(npairs[d]), int(pmax[d])
             # the point form costs 2 gathers per pair against one per stored non-zero; long lists
             # (millions of points per cell on coarse levels of large scenes) stay with the Gram
@@ -520,12 +538,7 @@ class Reconstruction(DualMesher):
             if lv.mf:
                 self._assemble_mf(lv, d)
             if not lv.mf or self.keep_csr:
-                # 2-byte column deltas where every |column - row| fits and the solver reads them
-                # (the launches that stage the vector in shared memory)
-                mode = self.solver.mode
-                delta_ok = bool(span[d] <= 32767 and mode is not None and
-                                L.load().ngs_pcg_window(lv.n, lv.nnz, lv.band, mode) == 1)
-                self._assemble_csr(lv, d, delta_ok)
+                self._assemble_csr(lv, d)
         self._mark("assembly")
         return self
 
@@ -551,9 +564,8 @@ class Reconstruction(DualMesher):
         """Screening weight of level d (reconstructor.py:122: alpha * (1/4)^d)."""
         return 0.25 ** d * self.alpha
 
-    def _assemble_csr(self, lv: Level, d: int, delta_ok: bool):
+    def _assemble_csr(self, lv: Level, d: int):
         st = L.stream()
-        lv.delta_ok = delta_ok
         lv.cols = torch.empty(lv.nnz, dtype=torch.int32, device=self.dev)
         lv.vals64 = torch.empty(lv.nnz, dtype=torch.float64, device=self.dev)
         lv.diag_slot = torch.empty(lv.n, dtype=torch.int64, device=self.dev)
@@ -571,16 +583,28 @@ class Reconstruction(DualMesher):
             lv.group = (keys, order)          # reused by the screening RHS terms of this level
             L.call("ngs_screen_gram_grouped", L.ptr(lv.rows), L.ptr(lv.phi), self.n, None, L.ptr(order),
                    L.ptr(keys), L.ptr(lv.masks), L.ptr(lv.rowptr), self._screen_scale(d), L.ptr(lv.vals64), st)
-        if lv.delta_ok:
-            # 2-byte column deltas for the solver's SpMV (6 instead of 8 bytes per non-zero)
-            lv.col_delta = torch.empty(lv.nnz, dtype=torch.int16, device=self.dev)
-            L.call("ngs_csr_col_delta", L.ptr(lv.rowptr), L.ptr(lv.cols), lv.n, L.ptr(lv.col_delta), st)
-        lv.vals32 = torch.empty(lv.nnz, dtype=torch.float32, device=self.dev)
         inv_diag = torch.empty(lv.n, dtype=torch.float32, device=self.dev)
-        L.call("ngs_finish_system", L.ptr(lv.vals64), lv.nnz, L.ptr(lv.diag_slot), lv.n, L.ptr(lv.vals32),
-               L.ptr(inv_diag), st)
+        if lv.pk_start is not None and not lv.mf:
+            # the solver's copy: values in its precision, 2-byte column deltas where every |column - row| fits
+            mode, wide = self.solver.mode, self.pk_wide(lv)
+            lv.pk_vals = torch.empty(lv.pk_units * 32, dtype=torch.float32 if mode == L.PCG_MIXED else torch.float64,
+                                     device=self.dev)
+            lv.pk_cols = torch.empty(L.load().ngs_pcg_pack_col_words(lv.n, lv.pk_units, wide), dtype=torch.int32,
+                                     device=self.dev)
+            L.call("ngs_pcg_pack_fill", L.ptr(lv.rowptr), L.ptr(lv.cols), L.ptr(lv.vals64), lv.n, L.ptr(lv.pk_start), wide,
+                   mode, L.ptr(lv.pk_vals), L.ptr(lv.pk_cols), st)
+            L.call("ngs_csr_inv_diag", L.ptr(lv.vals64), L.ptr(lv.diag_slot), lv.n, L.ptr(inv_diag), st)
+        else:
+            lv.vals32_ = torch.empty(lv.nnz, dtype=torch.float32, device=self.dev)
+            L.call("ngs_finish_system", L.ptr(lv.vals64), lv.nnz, L.ptr(lv.diag_slot), lv.n, L.ptr(lv.vals32_),
+                   L.ptr(inv_diag), st)
         if not lv.mf:
             lv.inv_diag = inv_diag
+
+    @staticmethod
+    def pk_wide(lv: Level) -> int:
+        """1 where the level's packed columns take 4 bytes."""
+        return int(not 0 < lv.band <= 32767)
 
     def mf_operator(self, lv: Level, d: int) -> "L.PcgOperator":
         """The C-ABI description of a matrix-free level (scratch for the per-point products included)."""
@@ -680,11 +704,15 @@ class Reconstruction(DualMesher):
         else:
             sysd.nnz = lv.nnz
             sysd.rowptr, sysd.cols = lv.rowptr.data_ptr(), lv.cols.data_ptr()
-            sysd.vals32, sysd.vals64 = lv.vals32.data_ptr(), lv.vals64.data_ptr()
-            b32 = lv.rhs.float()
-            sysd.b32 = b32.data_ptr()
-            sysd.col_delta = lv.col_delta.data_ptr() if lv.col_delta is not None else None
-            sysd.band = lv.band
+            sysd.vals64 = lv.vals64.data_ptr()
+            if lv.pk_vals is not None:
+                sysd.pk_start, sysd.pk_vals, sysd.pk_cols = (t.data_ptr() for t in (lv.pk_start, lv.pk_vals, lv.pk_cols))
+                sysd.pk_units, sysd.pk_wide = lv.pk_units, self.pk_wide(lv)
+                b32 = None
+            else:
+                sysd.vals32, sysd.band = lv.vals32.data_ptr(), lv.band
+                b32 = lv.rhs.float()
+                sysd.b32 = b32.data_ptr()
         sysd.b64 = lv.rhs.data_ptr()
         sysd.x32, sysd.x64 = lv.x32.data_ptr(), lv.x64.data_ptr()
         cfg = item.cfg
