@@ -528,6 +528,65 @@ int ngs_ddi_backward(const float* src, const float* tgt, const int64_t* rel_pos,
                      const float* dfdf, const float* grad_p, const float* grad_q, int64_t n_pairs, int C, int R,
                      float* grad_src, float* grad_tgt, ngs_stream s);
 
+/* ======================================================================= learned-basis terms
+ * ref: jspsr/bases/additive.py:55-414.  Per axis B(x) = sum_k m_k q_k(x), coefficients float
+ * [voxels, 3 C] (component-major, axis-minor).  Ids, rows and offsets are the caller's responsibility. */
+enum { NGS_COMP_POWER = 0, NGS_COMP_SIN = 1, NGS_COMP_BEZIER = 2 };
+typedef struct ngs_basis_comps {
+  int32_t count;             /* 1 .. 32 */
+  int32_t kind[32];          /* x^a; sin(a x + b); the quadratic B-spline, times two */
+  float a[32], b[32];
+} ngs_basis_comps;
+
+/* Values per axis f [m, 3] at x [m, 3] with a row of coefficients each, and the rows' gradient. */
+int ngs_basis_axes(const ngs_basis_comps* comps, const float* coef, const float* x, int64_t m, float* f, ngs_stream s);
+int ngs_basis_axes_grad(const ngs_basis_comps* comps, const float* x, const float* grad, int64_t m, float* gcoef,
+                        ngs_stream s);
+/* Values phi [n, 27] of the slots of every point (rows [n, 27], -1: none; local [n, 27, 3]); the gradient adds
+ * dL/dB of a slot, lam[row] pa[point] + xs[row] pb[point], into gcoef. */
+int ngs_basis_phi(const ngs_basis_comps* comps, const float* coef, const int32_t* rows, const float* local,
+                  int64_t n_points, float* phi, ngs_stream s);
+int ngs_basis_phi_grad(const ngs_basis_comps* comps, const float* coef, const int32_t* rows, const float* local,
+                       int64_t n_points, const double* lam, const double* xs, const double* pa, const double* pb,
+                       float* gcoef, ngs_stream s);
+
+typedef struct ngs_basis_pair_term {
+  const float *ff, *dd;      /* [C, C, R] tables, scaled by fscale and dscale */
+  const float *cs, *ct;      /* coefficients of the sources' and of the targets' voxels */
+  const int64_t* sid;        /* [pairs] */
+  const void* tid;           /* [pairs] int64, or int32 (tid32) */
+  const float* rel;          /* [pairs, 3]: table index round(rel + add), 0 outside */
+  int64_t pairs;
+  float fscale, dscale, add;
+  int32_t C, R, tid32, transposed;
+  double* out;               /* grad 0: the value of every pair, or y[source] -= value x[target] */
+  const double* x;           /* (transposed: y[target] -= value x[source]) */
+  double* y;
+  const double *lam, *xs;    /* grad 1: dL/dvalue = -lam[source] xs[target], added into gs and gt */
+  float *gs, *gt;            /* (either may be null) */
+} ngs_basis_pair_term;
+int ngs_basis_pairs_fit(int C, int R);       /* 1 where ngs_basis_pairs takes such tables */
+int ngs_basis_pairs(const ngs_basis_pair_term* term, int grad, ngs_stream s);
+
+typedef struct ngs_basis_div_term {
+  const float* f[32];        /* per component: tables of `len` entries, index round(rel mul + add) */
+  const float* df[32];
+  const float *coef, *data, *rel;   /* targets' coefficients; data [voxels, 3]; rel [pairs, 3] */
+  const int64_t *vid, *tid;  /* [pairs]: data voxel, target */
+  int64_t pairs;
+  int32_t C, len;
+  float mul, add, scale, pad_;
+  double* b;                 /* grad 0: b[target] += value */
+  const double* lam;         /* grad 1: gradient of lam[target] value, added into gcoef and gdata */
+  float *gcoef, *gdata;      /* (either may be null) */
+} ngs_basis_div_term;
+int ngs_basis_divergence(const ngs_basis_div_term* term, int grad, ngs_stream s);
+
+/* out[p] = sum over the slots of phi x[row]; out[row] += scale phi w[p]. */
+int ngs_point_sum64(const float* phi, const int32_t* rows, int64_t n, const double* x, double* out, ngs_stream s);
+int ngs_point_spread64(const float* phi, const int32_t* rows, int64_t n, const double* w, double scale, double* out,
+                       ngs_stream s);
+
 /* ======================================================================= marching cubes
  * ref: csrc/marching_cubes/primal_mc.cu:170-235 (marching_cubes_sparse), dual_mc.cu:135-189
  * (dual_marching_cubes_sparse), dual_mc_inds.cu:143-182 (dual_marching_cubes_indices).

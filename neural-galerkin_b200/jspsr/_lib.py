@@ -52,6 +52,26 @@ class PcgSystem(C.Structure):
                 ("pk_pad_", C.c_int32)]
 
 
+COMP_POWER, COMP_SIN, COMP_BEZIER = 0, 1, 2
+
+
+class BasisComps(C.Structure):
+    _fields_ = [("count", C.c_int32), ("kind", C.c_int32 * 32), ("a", C.c_float * 32), ("b", C.c_float * 32)]
+
+
+class BasisPairTerm(C.Structure):
+    _fields_ = [("ff", vp), ("dd", vp), ("cs", vp), ("ct", vp), ("sid", vp), ("tid", vp), ("rel", vp),
+                ("pairs", C.c_int64), ("fscale", C.c_float), ("dscale", C.c_float), ("add", C.c_float),
+                ("C", C.c_int32), ("R", C.c_int32), ("tid32", C.c_int32), ("transposed", C.c_int32), ("out", vp),
+                ("x", vp), ("y", vp), ("lam", vp), ("xs", vp), ("gs", vp), ("gt", vp)]
+
+
+class BasisDivTerm(C.Structure):
+    _fields_ = [("f", vp * 32), ("df", vp * 32), ("coef", vp), ("data", vp), ("rel", vp), ("vid", vp), ("tid", vp),
+                ("pairs", C.c_int64), ("C", C.c_int32), ("len", C.c_int32), ("mul", C.c_float), ("add", C.c_float),
+                ("scale", C.c_float), ("pad_", C.c_float), ("b", vp), ("lam", vp), ("gcoef", vp), ("gdata", vp)]
+
+
 class PcgConfig(C.Structure):
     _fields_ = [("mode", C.c_int), ("max_iter", C.c_int), ("tol", C.c_double), ("res_fix", C.c_int),
                 ("replace_every", C.c_int), ("blocks", C.c_int), ("timeout_s", C.c_double)]
@@ -167,6 +187,15 @@ _SIGS = {
     "ngs_screened_multiplication": ([H, vp, vp, C.c_int, vp, vp, vp, vp, vp, vp, vp, i64, vp, vp], C.c_int),
     "ngs_screened_multiplication_backward": ([H, vp, vp, C.c_int, vp, vp, vp, vp, vp, vp, vp, i64, vp, vp, vp,
                                               vp, vp], C.c_int),
+    "ngs_basis_axes": ([C.POINTER(BasisComps), vp, vp, i64, vp, vp], C.c_int),
+    "ngs_basis_axes_grad": ([C.POINTER(BasisComps), vp, vp, i64, vp, vp], C.c_int),
+    "ngs_basis_phi": ([C.POINTER(BasisComps), vp, vp, vp, i64, vp, vp], C.c_int),
+    "ngs_basis_phi_grad": ([C.POINTER(BasisComps), vp, vp, vp, i64, vp, vp, vp, vp, vp, vp], C.c_int),
+    "ngs_basis_pairs_fit": ([C.c_int, C.c_int], C.c_int),
+    "ngs_basis_pairs": ([C.POINTER(BasisPairTerm), C.c_int, vp], C.c_int),
+    "ngs_basis_divergence": ([C.POINTER(BasisDivTerm), C.c_int, vp], C.c_int),
+    "ngs_point_sum64": ([vp, vp, i64, vp, vp, vp], C.c_int),
+    "ngs_point_spread64": ([vp, vp, i64, vp, f64, vp, vp], C.c_int),
     "ngs_ddi_forward": ([vp, vp, vp, vp, vp, i64, C.c_int, C.c_int, vp, vp, vp], C.c_int),
     "ngs_ddi_backward": ([vp, vp, vp, vp, vp, vp, vp, i64, C.c_int, C.c_int, vp, vp, vp], C.c_int),
     "ngs_primal_mc_count": ([vp, i64, C.c_int, vp, vp], C.c_int),

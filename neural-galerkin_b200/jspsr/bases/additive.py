@@ -6,6 +6,7 @@ forms run in the DDI kernels (``ngs_ddi_forward / _backward``) behind ``DDIFunc`
 """
 from __future__ import annotations
 
+import ctypes as C
 from functools import lru_cache
 from typing import List, Union
 
@@ -15,7 +16,9 @@ import torch
 from .abc import BaseBasis
 from .additive_components import *          # noqa: F401,F403  (component names usable in basis specs)
 from .additive_components import AdditiveComponent, Bezier, Power, Sinusoid, SinPeaks, Product
+from .additive_terms import AXES_CHUNK, axes_table
 from . import tables as T
+from .. import _lib as L
 from .. import ext
 
 
@@ -44,11 +47,19 @@ class EvalFunc(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, xyz, coeffs, feat_ids, components):
+        table = axes_table(components, xyz, coeffs, feat_ids)
         with torch.no_grad():
-            out = 0
-            for ci, comp in enumerate(components):
-                out = out + comp.evaluate(xyz) * coeffs[feat_ids, 3 * ci:3 * ci + 3]
+            if table is not None:
+                out = torch.empty(xyz.shape, device=xyz.device)
+                for k in range(0, xyz.shape[0], AXES_CHUNK):
+                    rows, x = coeffs[feat_ids[k:k + AXES_CHUNK]], xyz[k:k + AXES_CHUNK].contiguous()
+                    L.call("ngs_basis_axes", C.byref(table), L.ptr(rows), L.ptr(x), x.shape[0], L.ptr(out[k:]), L.stream())
+            else:
+                out = 0
+                for ci, comp in enumerate(components):
+                    out = out + comp.evaluate(xyz) * coeffs[feat_ids, 3 * ci:3 * ci + 3]
         ctx.save_for_backward(xyz, feat_ids)
+        ctx.table = table
         ctx.components, ctx.n = components, coeffs.size(0)
         return out
 
@@ -56,6 +67,14 @@ class EvalFunc(torch.autograd.Function):
     def backward(ctx, grad):
         xyz, ids = ctx.saved_tensors
         with torch.no_grad():
+            if ctx.table is not None and grad.dtype == torch.float32:
+                out = torch.zeros((ctx.n, 3 * len(ctx.components)), device=xyz.device)
+                for k in range(0, xyz.shape[0], AXES_CHUNK):
+                    x, gk = xyz[k:k + AXES_CHUNK].contiguous(), grad[k:k + AXES_CHUNK].contiguous()
+                    g = torch.empty((x.shape[0], out.shape[1]), device=x.device)
+                    L.call("ngs_basis_axes_grad", C.byref(ctx.table), L.ptr(x), L.ptr(gk), x.shape[0], L.ptr(g), L.stream())
+                    out.index_add_(0, ids[k:k + AXES_CHUNK], g)
+                return None, out, None, None
             g = [_scatter_sum(grad * comp.evaluate(xyz), ids, ctx.n) for comp in ctx.components]
         return None, torch.cat(g, dim=1), None, None
 

@@ -40,6 +40,7 @@ import torch
 
 from .. import _lib as L
 from ..bases import tables as TB
+from ..bases.additive_terms import AdditiveTerms
 from ._hash_backend import VoxelLevel
 from .pipeline import Reconstruction, parse_solver
 
@@ -307,6 +308,32 @@ def _assemble_level(basis, shape: ShapeGeometry, d: int, feats, normal_data, x_c
     return sysm, b
 
 
+def _assemble_level_terms(terms, shape: ShapeGeometry, d: int, coefs, normal_data, coarse):
+    """``_assemble_level`` with the basis terms of ``bases.additive_terms``; coarse: e -> (solution, its field at
+    the points)."""
+    geo = shape.levels[d]
+    sf = 0.25 ** d
+    vals64 = terms.stiffness(geo, coefs[d])
+    b = torch.zeros(geo.n, dtype=torch.float64, device=vals64.device)
+    for dd in shape.data_levels:
+        terms.divergence(geo, dd, coefs[d], normal_data[dd], b)
+    phi = None
+    if shape.xyz is not None:
+        phi = terms.phi(geo, coefs[d])
+        keys, order = geo.group
+        L.call("ngs_screen_gram_grouped", L.ptr(geo.pt_rows), L.ptr(phi), shape.xyz.shape[0], L.ptr(shape.alpha),
+               L.ptr(order), L.ptr(keys), L.ptr(geo.masks), L.ptr(geo.rowptr), sf, L.ptr(vals64), L.stream())
+        w = shape.alpha_delta.double()
+        if coarse:
+            w = w - shape.alpha.double() * sum(chi for _, chi in coarse.values())
+        terms.point_spread(phi, geo, w, sf, b)
+    for e, (xe, _) in coarse.items():
+        terms.couple(geo, shape.levels[e], coefs[d], coefs[e], xe, b, False)
+    sysm = _finish(geo, vals64)
+    sysm.phi = phi
+    return sysm, b
+
+
 def shape_stride(shape: ShapeGeometry, d: int) -> int:
     return 1 << d
 
@@ -322,22 +349,32 @@ class GalerkinSolve(torch.autograd.Function):
         S = len(shapes)
         systems = [dict() for _ in range(S)]
         xs = [dict() for _ in range(S)]
+        terms = AdditiveTerms.of(basis, shapes, feats, normals)
         with torch.no_grad():
             depths = shapes[0].order
+            if terms is not None:
+                coefs = [{d: terms.coefficients(feats[s][d]) for d in depths} for s in range(S)]
+                fields = [dict() for _ in range(S)]
             for d in depths:
                 jobs = []
                 for s in range(S):
-                    coarse = {e: (xs[s][e], systems[s][e].phi) for e in xs[s]}
-                    sysm, b = _assemble_level(basis, shapes[s], d, feats[s], normals[s], coarse)
+                    if terms is not None:
+                        coarse = {e: (xs[s][e], fields[s].get(e)) for e in xs[s]}
+                        sysm, b = _assemble_level_terms(terms, shapes[s], d, coefs[s], normals[s], coarse)
+                    else:
+                        coarse = {e: (xs[s][e], systems[s][e].phi) for e in xs[s]}
+                        sysm, b = _assemble_level(basis, shapes[s], d, feats[s], normals[s], coarse)
                     systems[s][d] = sysm
                     jobs.append((shapes[s].levels[d], sysm, b))
                 sol, status = solve_levels(jobs, spec)
                 for s in range(S):
                     xs[s][d] = sol[s]
+                    if terms is not None and shapes[s].xyz is not None and d != depths[-1]:
+                        fields[s][d] = terms.point_field(systems[s][d].phi, shapes[s].levels[d], sol[s])
                     shapes[s].stats[d] = dict(iters=int(status[s][0]), status=int(status[s][1]), resid=float(status[s][4]),
                                               bnorm=float(status[s][5]))
         ctx.basis, ctx.shapes, ctx.spec, ctx.layout = basis, shapes, spec, layout
-        ctx.systems, ctx.xs = systems, xs
+        ctx.systems, ctx.xs, ctx.terms = systems, xs, terms
         ctx.save_for_backward(*[t for t in tensors if t is not None])
         ctx.has = [t is not None for t in tensors]
         out = []
@@ -361,6 +398,9 @@ class GalerkinSolve(torch.autograd.Function):
                 gx[s][d] = (g.double() if g is not None else
                             torch.zeros(shapes[s].levels[d].n, dtype=torch.float64, device=shapes[s].levels[d].level.device))
         lam = [dict() for _ in range(S)]
+        terms = ctx.terms
+        if terms is not None:
+            coefs = [{d: terms.coefficients(feats[s][d].detach()) for d in shapes[s].order} for s in range(S)]
         # adjoint solves, finest level first; each pushes its correction's transpose to the coarser levels
         with torch.no_grad():
             for d in reversed(shapes[0].order):
@@ -371,6 +411,16 @@ class GalerkinSolve(torch.autograd.Function):
                     shape, geo = shapes[s], shapes[s].levels[d]
                     sf = 0.25 ** d
                     phi_d = ctx.systems[s][d].phi
+                    if terms is not None:
+                        w = None
+                        if phi_d is not None and geo.cross:
+                            w = shape.alpha.double() * terms.point_field(phi_d, geo, lam[s][d])
+                        for e in geo.cross:
+                            geo_e = shape.levels[e]
+                            terms.couple(geo, geo_e, coefs[s][d], coefs[s][e], lam[s][d], gx[s][e], True)
+                            if w is not None:
+                                terms.point_spread(ctx.systems[s][e].phi, geo_e, w, -sf, gx[s][e])
+                        continue
                     for e in geo.cross:
                         a = _cross_stiffness(basis, feats[s].get(d), feats[s].get(e), geo, shape.levels[e])
                         i, j, _ = geo.cross[e]
@@ -385,6 +435,11 @@ class GalerkinSolve(torch.autograd.Function):
         grad_tensors = [None] * len(tensors)
         need = [t is not None and ctx.needs_input_grad[4 + k] for k, t in enumerate(tensors)]
         if not any(need):
+            return (None, None, None, None) + tuple(grad_tensors)
+        if terms is not None:
+            for s in range(S):
+                _shape_vjp_terms(terms, shapes[s], layout, s, feats[s], normals[s], ctx.xs[s], lam[s], ctx.systems[s],
+                                 need, grad_tensors)
             return (None, None, None, None) + tuple(grad_tensors)
         with torch.enable_grad():
             for s in range(S):
@@ -462,6 +517,51 @@ def _shape_vjp(basis, shape: ShapeGeometry, layout, s, feats, normals, xs, lam, 
     for d, t in n_in.items():
         if t.requires_grad and gmap.get(id(t)) is not None:
             grad_tensors[nidx[d]] = gmap[id(t)]
+
+
+def _shape_vjp_terms(terms, shape: ShapeGeometry, layout, s, feats, normals, xs, lam, systems, need, grad_tensors):
+    """``_shape_vjp`` with the basis terms of ``bases.additive_terms``: every term adds into the gradients of the
+    coefficients, which go back through the features once."""
+    fidx, nidx = layout[s]
+    with torch.enable_grad():
+        f_in = {d: feats[d].detach().requires_grad_(need[fidx[d]]) for d in shape.order}
+        graph = {d: terms.coefficients(f_in[d]) for d in shape.order}
+    coefs = {d: c.detach() for d, c in graph.items()}
+    gcoef = {d: torch.zeros_like(coefs[d]) if need[fidx[d]] else None for d in shape.order}
+    gdata = {dd: torch.zeros_like(normals[dd], memory_format=torch.contiguous_format) if need[nidx[dd]] else None
+             for dd in shape.data_levels}
+    screen = shape.xyz is not None
+    if screen:
+        # coefficients of lambda_i and x_i in dL/dB_i(p): the same level and the coarser ones' fields, the target;
+        # the same level and the finer ones' adjoint fields
+        a, target = shape.alpha.double(), shape.alpha_delta.double()
+        pa, pb = {}, {}
+        total = 0
+        for d in shape.order:
+            total = total + terms.point_field(systems[d].phi, shape.levels[d], xs[d])
+            pa[d] = 0.25 ** d * (target - a * total)
+        total = 0
+        for d in reversed(shape.order):
+            total = total + 0.25 ** d * terms.point_field(systems[d].phi, shape.levels[d], lam[d])
+            pb[d] = -(a * total)
+    for d in shape.order:
+        geo, x, l = shape.levels[d], xs[d], lam[d]
+        if gcoef[d] is not None:
+            terms.pairs_grad(geo, geo, coefs[d], coefs[d], l, x, gcoef[d], gcoef[d])
+            if screen:
+                terms.phi_grad(geo, coefs[d], l, x, pa[d], pb[d], gcoef[d])
+        for dd in shape.data_levels:
+            if gcoef[d] is not None or gdata[dd] is not None:
+                terms.divergence_grad(geo, dd, coefs[d], normals[dd], l, gcoef[d], gdata[dd])
+        for e in geo.cross:
+            if gcoef[d] is not None or gcoef[e] is not None:
+                terms.pairs_grad(geo, shape.levels[e], coefs[d], coefs[e], l, xs[e], gcoef[d], gcoef[e])
+    for d in shape.order:
+        if gcoef[d] is not None:
+            grad_tensors[fidx[d]], = torch.autograd.grad(graph[d], f_in[d], gcoef[d])
+    for dd, g in gdata.items():
+        if g is not None:
+            grad_tensors[nidx[dd]] = g
 
 
 def _flatten(feats_list, normals_list, depths):
