@@ -946,6 +946,25 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_MIN_BLOCKS) pcg_batch_kernel(
   pcg_body<MODE, OPS, PCG_FORM_ANY>(b.sys[lo], blockIdx.x - b.start[lo], sy);
 }
 
+// Small systems of a batch that have one cluster size and one SpMV form: a cluster each, in one launch.  A system's
+// CTAs and their arithmetic are those of its launch alone.  One after another a level of four learned shapes took
+// 4 x 1.26 ms on 16 of the 148 SMs: all solves of a training step 30.2 -> 13.0 ms.
+constexpr int PCG_CLUSTER_BATCH = 16;
+struct PcgClusterBatch {
+  PcgArgs sys[PCG_CLUSTER_BATCH];
+};
+static_assert(sizeof(PcgClusterBatch) <= 32000, "batch arguments must fit the kernel parameter space");
+
+template <int MODE, int FORM>
+__global__ void __launch_bounds__(PCG_THREADS, PCG_MIN_BLOCKS)
+    pcg_cluster_batch_kernel(const __grid_constant__ PcgClusterBatch b) {
+  __shared__ double cred[8], bcast[4];
+  const PcgArgs& a = b.sys[blockIdx.x / cluster_size()];
+  ClusterSync sy{cluster_rank(), cluster_size(), cred, bcast, 0, 0ull, a.budget_ns, false};
+  pcg_body<MODE, PCG_OPS_CSR, FORM>(a, sy.rank, sy);
+  cluster_sync_all();
+}
+
 static size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Element sizes of a mode's workspace vectors: search vectors (p, s, u, w) and residual r.  The one
@@ -1065,6 +1084,9 @@ static int pcg_cluster_limit() {
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_DELTA>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_COLS>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED>));
+    limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_DELTA>));
+    limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_COLS>));
+    limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_PACKED>));
   }
   if (limit > PCG_CLUSTER_MAX) limit = PCG_CLUSTER_MAX;
   if (dev >= 0 && dev < 64) cached[dev] = limit > 0 ? limit : -1;
@@ -1148,15 +1170,34 @@ static void pcg_set_window(PcgArgs& a, int mode, int64_t band, int64_t nblocks) 
 
 static size_t pcg_win_smem(const PcgArgs& a) { return a.win_cap > 0 ? PCG_WIN_BYTES : 0; }
 
-// One cluster of `csize` CTAs solves the system (an ordinary launch: the hardware places the whole
-// cluster at once, so the cluster barrier needs no cooperative launch).
-static int launch_cluster(PcgArgs& a, int mode, int csize, cudaStream_t st) {
-  a.nblocks = (unsigned int)csize;
-  cudaMemsetAsync(a.count, 0, 8 * sizeof(unsigned int), st);
+// The specialised cluster kernels of a system (alone, in a batch), or the general one with batch null.
+struct PcgClusterKernels {
+  const void *solo, *batch;
+};
+
+template <int MODE>
+static PcgClusterKernels pcg_cluster_forms(const PcgArgs& a) {
+  if (a.pk_start) return {(const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED>,
+                          (const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_PACKED>};
+  if (a.cols16) return {(const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_DELTA>,
+                        (const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_DELTA>};
+  return {(const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_COLS>,
+          (const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_COLS>};
+}
+
+static PcgClusterKernels pcg_cluster_kernels_of(const PcgArgs& a, int mode) {
+  if (mode == NGS_PCG_REFERENCE || a.mf || a.evict_first || (a.pk_start && a.pk_wide))
+    return {pcg_cluster_kernel_of(mode, a.mf != 0), nullptr};
+  return mode == NGS_PCG_MIXED ? pcg_cluster_forms<NGS_PCG_MIXED>(a) : pcg_cluster_forms<NGS_PCG_FP64>(a);
+}
+
+// `count` clusters of `csize` CTAs (an ordinary launch: the hardware places a whole cluster at once, so the cluster
+// barrier needs no cooperative launch, and clusters do not wait for one another).
+static int launch_clusters(const void* f, void* params, int csize, int count, size_t smem, cudaStream_t st) {
   cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3((unsigned)csize);
+  lc.gridDim = dim3((unsigned)(csize * count));
   lc.blockDim = dim3(PCG_THREADS);
-  lc.dynamicSmemBytes = pcg_win_smem(a);
+  lc.dynamicSmemBytes = smem;
   lc.stream = st;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -1165,23 +1206,17 @@ static int launch_cluster(PcgArgs& a, int mode, int csize, cudaStream_t st) {
   attr.val.clusterDim.z = 1;
   lc.attrs = &attr;
   lc.numAttrs = 1;
-  void* args[] = {&a};
+  void* args[] = {params};
   ngs_count_launch();
-  const void* f = pcg_cluster_kernel_of(mode, a.mf != 0);
-  if (!a.mf && a.pk_start && !a.pk_wide && !a.evict_first && (mode == NGS_PCG_MIXED || mode == NGS_PCG_FP64)) {
-    f = mode == NGS_PCG_MIXED ? (const void*)pcg_cluster_form_kernel<NGS_PCG_MIXED, PCG_FORM_PACKED>
-                              : (const void*)pcg_cluster_form_kernel<NGS_PCG_FP64, PCG_FORM_PACKED>;
-  } else if (!a.mf && !a.pk_start && !a.evict_first && (mode == NGS_PCG_MIXED || mode == NGS_PCG_FP64)) {
-    if (mode == NGS_PCG_MIXED)
-      f = a.cols16 ? (const void*)pcg_cluster_form_kernel<NGS_PCG_MIXED, PCG_FORM_DELTA>
-                   : (const void*)pcg_cluster_form_kernel<NGS_PCG_MIXED, PCG_FORM_COLS>;
-    else
-      f = a.cols16 ? (const void*)pcg_cluster_form_kernel<NGS_PCG_FP64, PCG_FORM_DELTA>
-                   : (const void*)pcg_cluster_form_kernel<NGS_PCG_FP64, PCG_FORM_COLS>;
-  }
   const cudaError_t e = cudaLaunchKernelExC(&lc, f, args);
-  if (e != cudaSuccess) return ngs_set_cuda_error(e);
-  return NGS_OK;
+  return e == cudaSuccess ? NGS_OK : ngs_set_cuda_error(e);
+}
+
+// One cluster of `csize` CTAs solves the system.
+static int launch_cluster(PcgArgs& a, int mode, int csize, cudaStream_t st) {
+  a.nblocks = (unsigned int)csize;
+  cudaMemsetAsync(a.count, 0, 8 * sizeof(unsigned int), st);
+  return launch_clusters(pcg_cluster_kernels_of(a, mode).solo, &a, csize, 1, pcg_win_smem(a), st);
 }
 
 // Zero a system's status record: the kernel's status writes are maxima over it, and an empty system
@@ -1389,9 +1424,31 @@ extern "C" int ngs_pcg_solve_batch(const ngs_pcg_batch_item* items, int n_items,
     total += (unsigned)blocks;
   }
   for (int k = 0; k < nempty; k++) pcg_clear_status(items[empty[k]].info_dev, items[empty[k]].resid_dev, st);
+  for (int k = 0; k < nsmall; k++) pcg_clear_status(small[k].info, small[k].resid, st);
+  static thread_local PcgClusterBatch group;
   for (int k = 0; k < nsmall; k++) {
-    pcg_clear_status(small[k].info, small[k].resid, st);
-    const int rc = launch_cluster(small[k], mode, small_size[k], st);
+    const int csize = small_size[k];
+    if (csize == 0) continue;                // launched with an earlier system
+    const PcgClusterKernels f = pcg_cluster_kernels_of(small[k], mode);
+    const size_t smem = pcg_win_smem(small[k]);
+    int like[PCG_CLUSTER_BATCH], count = 0;
+    for (int j = k; j < nsmall && count < PCG_CLUSTER_BATCH; j++)
+      if (f.batch && small_size[j] == csize && pcg_win_smem(small[j]) == smem &&
+          pcg_cluster_kernels_of(small[j], mode).batch == f.batch)
+        like[count++] = j;
+    int rc;
+    if (count > 1) {
+      for (int j = 0; j < count; j++) {
+        PcgArgs& a = small[like[j]];
+        a.nblocks = (unsigned int)csize;
+        cudaMemsetAsync(a.count, 0, 8 * sizeof(unsigned int), st);
+        group.sys[j] = a;
+        small_size[like[j]] = 0;
+      }
+      rc = launch_clusters(f.batch, &group, csize, count, smem, st);
+    } else {
+      rc = launch_cluster(small[k], mode, csize, st);
+    }
     if (rc != NGS_OK) return rc;
   }
   if (b.nsys == 0) return NGS_OK;

@@ -61,24 +61,37 @@ def pack(m, mode, wide):
 
 
 def solve(m, mode, wide, blocks=0):
+    item, x64, keep = batch_item(m, mode, wide, blocks)
+    L.call("ngs_pcg_solve", C.byref(item.sys), C.byref(item.cfg), item.ws, item.ws_bytes, item.info_dev, item.resid_dev,
+           L.stream())
+    info = keep[-1]
+    assert int(info[1]) == 0, int(info[1])
+    return x64
+
+
+def batch_item(m, mode, wide, blocks=0, packed=True):
     start, vals, cols = pack(m, mode, wide)
     dinv = torch.empty(m["n"], device=DEV)
     L.call("ngs_csr_inv_diag", L.ptr(m["vals"]), L.ptr(m["diag"]), m["n"], L.ptr(dinv), L.stream())
     x32, x64 = torch.empty(m["n"], device=DEV), torch.zeros(m["n"], dtype=torch.float64, device=DEV)
     info = torch.zeros(4, dtype=torch.int64, device=DEV)
     resid = torch.zeros(2, dtype=torch.float64, device=DEV)
-    s, cfg = L.PcgSystem(), L.PcgConfig()
+    item = L.PcgBatchItem()
+    s, cfg = item.sys, item.cfg
     s.n, s.nnz, s.rowptr, s.cols, s.vals64 = m["n"], m["nnz"], m["ptr"].data_ptr(), m["cols"].data_ptr(), m["vals"].data_ptr()
     s.inv_diag, s.b64, s.x32, s.x64 = dinv.data_ptr(), m["b"].data_ptr(), x32.data_ptr(), x64.data_ptr()
-    s.pk_start, s.pk_vals, s.pk_cols = start.data_ptr(), vals.data_ptr(), cols.data_ptr()
-    s.pk_units, s.pk_wide = int(start[-1]), wide
+    v32 = m["vals"].float()
+    if packed:
+        s.pk_start, s.pk_vals, s.pk_cols = start.data_ptr(), vals.data_ptr(), cols.data_ptr()
+        s.pk_units, s.pk_wide = int(start[-1]), wide
+    else:
+        s.vals32 = v32.data_ptr()
     cfg.mode, cfg.max_iter, cfg.tol, cfg.res_fix = mode, 5000, TOL, 0
     cfg.replace_every, cfg.blocks, cfg.timeout_s = 50, blocks, 10.0
     nb = L.load().ngs_pcg_workspace_bytes(m["n"], mode)
     ws = torch.empty(nb, dtype=torch.uint8, device=DEV)
-    L.call("ngs_pcg_solve", C.byref(s), C.byref(cfg), L.ptr(ws), nb, L.ptr(info), L.ptr(resid), L.stream())
-    assert int(info[1]) == 0, int(info[1])
-    return x64
+    item.ws, item.ws_bytes, item.info_dev, item.resid_dev = ws.data_ptr(), nb, info.data_ptr(), resid.data_ptr()
+    return item, x64, (m, start, vals, cols, dinv, x32, v32, resid, ws, info)
 
 
 def residual(m, x):
@@ -127,3 +140,24 @@ def test_packed_entries(n, per_row, wide):
         k = ptr[row + 1] - ptr[row]
         assert np.array_equal(got_v[:k], v[ptr[row]:ptr[row + 1]]) and np.array_equal(got_c[:k], c[ptr[row]:ptr[row + 1]])
         assert not got_v[k:].any() and (got_c[k:] == row).all()
+
+
+@pytest.mark.parametrize("mode", [L.PCG_MIXED, L.PCG_FP64])
+def test_clusters_of_a_batch_equal_solo_solves(mode):
+    """Small systems of one batch share launches by cluster size and form (at most 16 a launch): every solution is
+    bit for bit that of its solo solve, with forms and sizes mixed and a system without a batch partner."""
+    lib = L.load()
+    shapes = [(2000, 20)] * 18 + [(1, 0), (300, 5), (9001, 40), (9002, 40), (0, 0), (4000, 60)]
+    systems = [system(n, per, 7 + k) for k, (n, per) in enumerate(shapes) if n]
+    kinds = [(k % 5 == 4, k % 3 != 1) for k in range(len(systems))]                  # 4-byte columns, packed
+    assert len({lib.ngs_pcg_cluster_size(m["n"], m["nnz"], mode) for m in systems}) > 2
+    assert all(lib.ngs_pcg_cluster_size(m["n"], m["nnz"], mode) > 0 for m in systems)
+    items = [batch_item(m, mode, int(w), packed=p) for m, (w, p) in zip(systems, kinds)]
+    arr = (L.PcgBatchItem * len(items))(*[i[0] for i in items])
+    L.call("ngs_pcg_solve_batch", arr, len(items), L.stream())
+    for m, (w, p), (_, x, keep) in zip(systems, kinds, items):
+        assert int(keep[-1][1]) == 0 and residual(m, x) <= 1.01 * TOL
+        solo, y, kept = batch_item(m, mode, int(w), packed=p)
+        L.call("ngs_pcg_solve", C.byref(solo.sys), C.byref(solo.cfg), solo.ws, solo.ws_bytes, solo.info_dev,
+               solo.resid_dev, L.stream())
+        assert torch.equal(x, y) and torch.equal(keep[-1], kept[-1])
