@@ -12,14 +12,16 @@
 // gradient is the same kernel over the transposed table with W[k]^T; the weight gradient is a GEMM
 // over the pairs of one offset (split over CTAs, partials reduced in a fixed order).
 //
-// Warp roles in the tile kernel (288 threads): warps 0-7 gather tiles into a ring of shared-memory
-// stages (two threads per tile row) and run the epilogue (warp w reads TMEM lanes 32(w%4).. = tile
-// rows, column half w/4); warp 8 allocates TMEM and one of its lanes issues the MMAs.  Stages are
-// handed over through mbarriers: "full" (256 producer arrivals after their stores and a proxy
-// fence) and "empty" (tcgen05.commit of the MMAs that read the stage).  Every wait is bounded; on timeout the kernel records NGS_ERR_TIMEOUT,
-// stops issuing, waits (bounded) for its MMAs and releases its TMEM before returning.
+// Warp roles of the gather GEMM: at "tiles through TMA" below.  In the tile kernel of the weight gradient (288
+// threads) warps 0-7 gather tiles into a ring of shared-memory stages and run the epilogue (warp w reads TMEM lanes
+// 32(w%4).. = tile rows, column half w/4); warp 8 allocates TMEM and one of its lanes issues the MMAs.  Stages are
+// handed over through mbarriers: "full" (arrivals after the stores and a proxy fence) and "empty" (tcgen05.commit of
+// the MMAs that read the stage).  Every wait is bounded; on timeout the kernel records NGS_ERR_TIMEOUT, stops
+// issuing, waits (bounded) for its copies and MMAs and releases its TMEM before returning.
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "ngs_common.cuh"
@@ -360,6 +362,187 @@ NGS_DEV void st16_row(void* out, bool f32, int bf16, int64_t off, const float (&
 
 }  // namespace conv
 
+// ----------------------------------------------------------------------------- tiles through TMA
+// The tile kernel with most of its stages' bytes moved by TMA: two warps issue the copies (a row gather moves four
+// rows of 128 bytes, zeros for rows and channels out of range, in the swizzled layout), one thread issues the MMAs,
+// and the four warps of the epilogue copy the tile's last rows with cp.async meanwhile.  Both ways of copying have a
+// rate of their own.  1.3M rows of 64 -> 64 channels, 27 offsets: 1,310 us with cp.async alone (the producers'
+// instructions, 270 a step and warp), 1,128 with one warp issuing all rows by TMA (50 cycles a gather), 772 with four,
+// 760 in this form.  What is left is the chain of a step through its barriers (620 us of it remain with no bytes
+// moved at all); L2 runs at 30 % and DRAM at 7 % of their rates.
+namespace conv {
+
+constexpr int TMA_THREADS = 224;         // warps 0 and 6: TMA, warp 1: MMAs, warps 2-5: cp.async, then epilogue
+constexpr int TMA_STAGES = 8;            // of the ring, at most
+
+NGS_DEV void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// Four rows of 128 bytes (the map's box: 64 elements, one row) at channel c.
+NGS_DEV void tma_gather4(uint32_t dst, const CUtensorMap* map, int c, int r0, int r1, int r2, int r3, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], "
+      "[%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+      "l"(map), "r"(c), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(smem_u32(bar))
+      : "memory");
+}
+NGS_DEV void tma_tile(uint32_t dst, const CUtensorMap* map, int c, int r, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(map), "r"(c), "r"(r), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// Every producer warp walks the steps for itself: next() finds its next step and returns the valid reduction elements
+// (0: no more).  Issue: issue(a, bar, w) starts TMA warp w's copies into the stage, t.tx[w] bytes in all; copy(a, w)
+// issues the cp.async of warp w of four.
+struct TmaShape {
+  int n, stages;
+  uint32_t stage_bytes, tx[2];
+  bool mn_major;
+};
+
+template <typename Setup, typename Next, typename Issue, typename Copy, typename Store>
+NGS_DEV void run_tile_tma(const TmaShape& t, uint8_t* smem, Setup& setup, Next& next, Issue& issue, Copy& copy, Store& store,
+                          int bf16, int* error) {
+  __shared__ uint64_t full_bar[TMA_STAGES], empty_bar[TMA_STAGES], done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag, any_step;
+  __shared__ int ksteps_of[TMA_STAGES];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int S = t.stages;
+  const uint32_t ncols_alloc = t.n <= 32 ? 32u : t.n <= 64 ? 64u : t.n <= 128 ? 128u : 256u;
+  if (tid == 0) {
+    for (int s = 0; s < S; s++) {
+      mbar_init(&full_bar[s], 6);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&done_bar, 2);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    abort_flag = 0;
+    any_step = 0;
+  }
+  if (warp == 1) tmem_alloc(&tmem_slot, ncols_alloc);
+  setup();
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  if (warp == 0 || warp == 6) {
+    const int w = warp == 6;
+    int st = 0, s = 0;
+    uint32_t parity = 1u;                        // of the round before this one
+    bool more = true;
+    while (more) {
+      const int valid = next();
+      more = valid > 0;
+      const bool go = s < S || mbar_wait(&empty_bar[st], parity, &abort_flag);
+      if (!__all_sync(0xffffffffu, go)) break;
+      if (lane == 0) {
+        if (w == 0) ksteps_of[st] = (valid + UK - 1) / UK;   // 0: no more steps
+        if (more && t.tx[w] > 0) mbar_expect(&full_bar[st], t.tx[w]);
+        else mbar_arrive(&full_bar[st]);
+      }
+      __syncwarp();
+      if (more) issue(smem + (size_t)st * t.stage_bytes, &full_bar[st], w);
+      s++;
+      if (++st == S) {
+        st = 0;
+        parity ^= 1u;
+      }
+    }
+    // after an abort the copies still land before the shared memory is given up (waits bounded again)
+    if (more && lane == 0)
+      for (int r = max(0, s - S); r < s; r++) {
+        int never = 0;
+        mbar_wait(&full_bar[r % S], (uint32_t)(r / S) & 1u, &never);
+      }
+  } else if (warp >= 2) {
+    // a step's copies are handed over while the next one's are in flight (the ring has two stages or more)
+    auto hand_over = [&](int st) {
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[st]);
+    };
+    int st = 0, s = 0, last = -1;
+    uint32_t parity = 1u;
+    bool more = true;
+    while (more) {
+      more = next() > 0;
+      const bool go = s < S || mbar_wait(&empty_bar[st], parity, &abort_flag);
+      if (!__all_sync(0xffffffffu, go)) break;
+      if (more) copy(smem + (size_t)st * t.stage_bytes, warp - 2);
+      cp_async_commit();
+      if (last >= 0) {
+        cp_async_wait<1>();
+        hand_over(last);
+      }
+      last = st;
+      s++;
+      if (++st == S) {
+        st = 0;
+        parity ^= 1u;
+      }
+    }
+    cp_async_wait<0>();
+    if (last >= 0) hand_over(last);
+  } else if (warp == 1 && lane == 0) {
+    const uint32_t idesc = t.mn_major ? f16_idesc_mn(BM, t.n, bf16) : f16_idesc(BM, t.n, bf16);
+    int st = 0;
+    uint32_t parity = 0u, accumulate = 0u;
+    for (;;) {
+      if (!mbar_wait(&full_bar[st], parity, &abort_flag)) break;
+      tc_fence_after();
+      const uint32_t a = smem_u32(smem + (size_t)st * t.stage_bytes), b = a + A_BYTES;
+      const int ks = ksteps_of[st];
+      if (ks == 0) break;
+      for (int kk = 0; kk < ks; kk++) {
+        umma_f16(tmem, t.mn_major ? mnmajor_sw128_desc(a + kk * 2048) : kmajor_sw128_desc(a + kk * 32),
+                 t.mn_major ? mnmajor_sw128_desc(b + kk * 2048) : kmajor_sw128_desc(b + kk * 32), idesc, accumulate);
+        accumulate = 1u;
+      }
+      umma_commit(&empty_bar[st]);
+      if (++st == S) {
+        st = 0;
+        parity ^= 1u;
+      }
+    }
+    any_step = (int)accumulate;
+    umma_commit(&done_bar);        // arrives once everything issued above has completed,
+    mbar_arrive(&done_bar);        // and here for any_step
+  }
+
+  if (warp >= 2 && warp < 6) {
+    // warp w reads TMEM lanes 32 (w % 4) ..: its tile rows
+    bool ok = mbar_wait(&done_bar, 0u, &abort_flag);
+    ok = __all_sync(0xffffffffu, ok) && !abort_flag;
+    tc_fence_after();
+    const int w = warp & 3, row = 32 * w + lane;
+    const bool any = any_step != 0;
+    for (int cc = 0; cc < t.n / 16; cc++) {
+      float v[16];
+      if (ok && any) {
+        tmem_ld16(tmem + ((uint32_t)(32 * w) << 16) + (uint32_t)(cc * 16), v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = 0.f;
+      }
+      if (ok) store(row, cc * 16, v);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_free(tmem, ncols_alloc);
+  }
+  if (tid == 0 && abort_flag) atomicExch(error, NGS_ERR_TIMEOUT);
+}
+
+}  // namespace conv
+
 // ----------------------------------------------------------------------------- gather GEMM (forward, input grad)
 // out[r, n] = sum over offsets k with table[r, k] = i >= 0 of sum_c x[i, c] * bt[k, n, c]
 // (forward: x = input features, bt = W[k]^T; input gradient: x = output gradient, table transposed,
@@ -380,89 +563,85 @@ struct GatherGemm {
   int stages;
   uint32_t stage_bytes;
   int* error;
+  int32_t oob;
 };
 
-__global__ void __launch_bounds__(conv::THREADS, 1) conv_gather_gemm_kernel(const __grid_constant__ GatherGemm g) {
+// Rows of a tile that are copied with cp.async (a multiple of 16), and the blocks an SM is to hold.  1.3M rows of
+// 64 -> 64 channels: 776, 767 and 800 us with 32, 48 and 64 rows; 907 with three blocks.
+constexpr int CP_ROWS = 48, TMA_ROWS = conv::BM - CP_ROWS;
+constexpr int CONV_PER_SM = 4;
+
+__global__ void __launch_bounds__(conv::TMA_THREADS) conv_gather_gemm_kernel(const __grid_constant__ GatherGemm g,
+                                                                            const __grid_constant__ CUtensorMap xmap,
+                                                                            const __grid_constant__ CUtensorMap bmap) {
   using namespace conv;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  __shared__ uint32_t act_mask[KMAX / 32];
-  __shared__ int act_list[KMAX];
-  __shared__ int n_act;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int64_t r0 = (int64_t)blockIdx.x * BM;
-  const int n0 = blockIdx.y * 256;
-  const int N = min(256, g.ncols - n0);
-  // the offsets with at least one pair in this tile (empty offsets cost nothing)
-  if (tid < KMAX / 32) act_mask[tid] = 0u;
-  __syncthreads();
-  if (tid < BM && r0 + tid < g.n_rows) {
-    const int32_t* t0 = g.table + (r0 + tid) * g.row_stride;
-#pragma unroll 9
-    for (int k = 0; k < g.K; k++) {
-      const unsigned any = __ballot_sync(__activemask(), __ldg(t0 + k * g.k_stride) >= 0);
-      if (any && (tid & 31) == 0) atomicOr(&act_mask[k >> 5], 1u << (k & 31));
-    }
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int c = 0;
-    for (int k = 0; k < g.K; k++)
-      if (act_mask[k >> 5] >> (k & 31) & 1u) act_list[c++] = k;
-    n_act = c;
-  }
-  __syncthreads();
-  const int nchunks = (g.kdim + BK - 1) / BK;
-  TileShape t{n_act * nchunks, N, g.stages, g.stage_bytes};
-
-  // eight producers per tile row, one 16-byte chunk each (a row's 128 bytes in one request), four rows
-  // per producer; the rows' table entries are read one offset ahead.  B rows likewise.  The bound is the
-  // producers' instructions (18 warps an SM, 9 cycles from one to the next), not the memory: 1.3M rows of
-  // 64 -> 64 channels took 1.67 ms with loads through registers, 1.64 with asynchronous copies alone,
-  // 1.31 once the ring's divisions and the variable-size form of the copies were gone.
-  const int prow = tid >> 3, pchunk = tid & 7;
-  const uint32_t at = sw128(prow, pchunk);            // 32 rows further on: 4 KB
-  const int32_t* const trow = g.table + (r0 + prow) * g.row_stride;
-  const int left = (int)min((int64_t)BM, g.n_rows - r0) - prow;
+  const int n0 = blockIdx.y * 256, rows = (int)min((int64_t)BM, g.n_rows - r0);
   const unsigned n_src = (unsigned)g.n_src;
-  const int kdim = g.kdim;
-  auto entries = [&](int i, int32_t (&src)[4]) {
-    const int32_t* tk = trow + act_list[i] * g.k_stride;
+  const uint32_t half = TMA_ROWS / 8 * 512;
+  TmaShape t{min(256, g.ncols - n0), g.stages, g.stage_bytes, {half + (uint32_t)min(256, g.ncols) * 128u, half}, false};
+
+  // entries of rows 4 lane .. 4 lane + 3 at an offset: `oob`, a row out of the map's range (zeros), for missing ones
+  const int32_t* const te = g.table + (r0 + 4 * lane) * g.row_stride;
+  const int left = rows - 4 * lane;
+  auto entries = [&](int k) {
+    int v[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) src[j] = 32 * j < left ? __ldg(tk + 32 * j * g.row_stride) : -1;
+    for (int j = 0; j < 4; j++) v[j] = j < left && k < g.K ? __ldg(te + j * g.row_stride + k * g.k_stride) : -1;
+    return make_int4(v[0], v[1], v[2], v[3]);
   };
-  int32_t src[4] = {-1, -1, -1, -1}, next[4] = {-1, -1, -1, -1};
-  int active = 0, c0 = 0;                             // the step's place in act_list and its first channel
-  if (tid < PRODUCERS && t.steps > 0) entries(0, src);
-  auto fill = [&](int s, uint8_t* a, uint8_t* b, int p) -> int {
-    const int k = act_list[active], e = c0 + pchunk * 8, valid = min(BK, kdim - c0);
-    const bool in = e < kdim;
-    if (c0 == 0 && active + 1 < n_act) entries(active + 1, next);
-    const uint16_t* xe = g.x + e;
-    const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+  // the offsets with at least one pair in this tile (empty offsets cost nothing), each in chunks of 64 channels; the
+  // next three offsets' entries are on their way meanwhile
+  int k = -1, c0 = g.kdim;
+  int4 src = make_int4(0, 0, 0, 0), ahead[3];
+  auto setup = [&] {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const bool have = in && (unsigned)src[j] < n_src;
-      cp_async16(sa + at + j * 4096, have ? xe + (int64_t)src[j] * kdim : g.x, have);
+    for (int i = 0; i < 3; i++) ahead[i] = entries(i);
+  };
+  auto next = [&]() -> int {
+    if (c0 + BK < g.kdim) {
+      c0 += BK;
+      return min(BK, g.kdim - c0);
     }
-    const uint16_t* bk = g.bt + ((int64_t)k * g.ncols + n0 + prow) * kdim;
-    for (int n = prow; n < N; n += 32) {
-      cp_async16(sb + at + (n - prow) * 128, in ? bk + e : g.bt, in);
-      bk += 32 * kdim;
-    }
-    c0 += BK;
-    if (c0 >= kdim) {
-      c0 = 0;
-      active++;
+    c0 = 0;
+    do {
+      if (++k >= g.K) return 0;
+      src = ahead[0];
+      ahead[0] = ahead[1];
+      ahead[1] = ahead[2];
+      ahead[2] = entries(k + 3);
+      src.x = (unsigned)src.x < n_src ? src.x : g.oob;
+      src.y = (unsigned)src.y < n_src ? src.y : g.oob;
+      src.z = (unsigned)src.z < n_src ? src.z : g.oob;
+      src.w = (unsigned)src.w < n_src ? src.w : g.oob;
+    } while (!__any_sync(0xffffffffu, src.x != g.oob || src.y != g.oob || src.z != g.oob || src.w != g.oob));
+    return min(BK, g.kdim);
+  };
+  auto issue = [&](uint8_t* a, uint64_t* bar, int w) {
+    const uint32_t sa = smem_u32(a);
+    if (w == 0 && lane == 31) tma_tile(sa + A_BYTES, &bmap, c0, k * g.ncols + n0, bar);
+    if (lane / (TMA_ROWS / 8) == w) tma_gather4(sa + lane * 512, &xmap, c0, src.x, src.y, src.z, src.w, bar);
+  };
+  // eight lanes per row, one 16-byte piece each
+  auto copy = [&](uint8_t* a, int w) {
+    const uint32_t sa = smem_u32(a);
+    const int piece = lane & 7, of4 = lane >> 3, e = c0 + piece * 8, quad0 = (TMA_ROWS + w * (CP_ROWS / 4)) / 4;
 #pragma unroll
-      for (int j = 0; j < 4; j++) src[j] = next[j];
+    for (int j = 0; j < CP_ROWS / 16; j++) {
+      const int x = __shfl_sync(0xffffffffu, src.x, quad0 + j), y = __shfl_sync(0xffffffffu, src.y, quad0 + j);
+      const int z = __shfl_sync(0xffffffffu, src.z, quad0 + j), u = __shfl_sync(0xffffffffu, src.w, quad0 + j);
+      const int32_t v = of4 < 2 ? (of4 == 0 ? x : y) : (of4 == 2 ? z : u);
+      const bool have = v != g.oob && e < g.kdim;
+      cp_async16(sa + sw128((quad0 + j) * 4 + of4, piece), have ? g.x + (int64_t)v * g.kdim + e : g.x, have);
     }
-    return valid;
   };
   auto store = [&](int row, int col, const float (&v)[16]) {
-    if (r0 + row < g.n_rows) st16_row(g.out, g.out_f32 != 0, g.bf16, (r0 + row) * g.ncols + n0 + col, v);
+    if (row < rows) st16_row(g.out, g.out_f32 != 0, g.bf16, (r0 + row) * g.ncols + n0 + col, v);
   };
-  run_tile<true>(t, smem, fill, store, g.bf16, g.error);
+  run_tile_tma(t, smem, setup, next, issue, copy, store, g.bf16, g.error);
 }
 
 // ----------------------------------------------------------------------------- weight gradient
@@ -881,6 +1060,28 @@ namespace {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+// The tensor map of `rows` rows of `width` 16-bit elements, in boxes of 64 elements and `box` rows, swizzled over 128
+// bytes, zeros out of range.  false where the driver refuses it.
+bool rows_map(CUtensorMap& map, const void* base, int64_t width, int64_t rows, int box) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<Encode>(fn);
+  }();
+  if (!encode) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)width * 2};
+  const cuuint32_t boxes[2] = {conv::BK, (cuuint32_t)box}, steps[2] = {1, 1};
+  return encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims, strides, boxes, steps,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Stages of the ring for an N-column tile, and the dynamic shared memory of the launch.
 void tile_plan(int n, int& stages, uint32_t& stage_bytes, size_t& smem) {
   const uint32_t nb = (uint32_t)((n + 7) / 8 * 8) * 128u;
@@ -1008,19 +1209,29 @@ static int conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_
   g.out_f32 = out_f32 || dtype == NGS_F32;
   g.bf16 = dtype == NGS_BF16;
   g.error = error_dev;
-  if (!ngs_conv_tensor_core_ok(kdim, ncols, dtype) || !aligned16(x) || !aligned16(bt) || !aligned16(out)) {
+  CUtensorMap xmap, bmap;
+  const int box = std::min(ncols, 256);
+  if (!ngs_conv_tensor_core_ok(kdim, ncols, dtype) || !aligned16(x) || !aligned16(bt) || !aligned16(out) ||
+      !rows_map(xmap, g.x, kdim, std::max<int64_t>(n_src, 1), 1) || !rows_map(bmap, bt, kdim, (int64_t)K * ncols, box)) {
     if (dtype == NGS_F32) return simt_gemm<float>(g, st);
     if (dtype == NGS_BF16) return simt_gemm<__nv_bfloat16>(g, st);
     return simt_gemm<__half>(g, st);
   }
-  size_t smem = 0;
-  tile_plan(ncols < 256 ? ncols : 256, g.stages, g.stage_bytes, smem);
-  if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
+  g.oob = n_src < 0x7fffffff ? (int32_t)std::max<int64_t>(n_src, 1) : -1;
+  // as many blocks on an SM as its shared memory and the tensor memory hold, up to CONV_PER_SM, of two stages or more
+  const size_t fixed = 1024;                                    // alignment of the first stage
+  g.stage_bytes = conv::A_BYTES + (uint32_t)((box * 128 + 1023) & ~1023);
+  for (int per_sm = std::min(CONV_PER_SM, 512 / std::max(box, 32)); per_sm >= 1; per_sm--) {
+    const size_t room = (227 << 10) / per_sm - 1536;            // the kernel's static arrays, the block's reserve
+    g.stages = fixed < room ? (int)std::min<size_t>((room - fixed) / g.stage_bytes, conv::TMA_STAGES) : 0;
+    if (g.stages >= 2) break;
+  }
+  const size_t smem = fixed + (size_t)g.stages * g.stage_bytes;
+  if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return ngs_set_cuda_error(cudaGetLastError());
   const dim3 grid((unsigned)((n_rows + conv::BM - 1) / conv::BM), (unsigned)((ncols + 255) / 256));
   ngs_count_launch();
-  conv_gather_gemm_kernel<<<grid, conv::THREADS, smem, st>>>(g);
+  conv_gather_gemm_kernel<<<grid, conv::TMA_THREADS, smem, st>>>(g, xmap, bmap);
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }
