@@ -376,6 +376,9 @@ int ngs_pcg_pack_fill(const int64_t* rowptr, const int32_t* cols, const double* 
                       const int64_t* start, int wide, int mode, void* pk_vals, int32_t* pk_cols, ngs_stream s);
 /* inv_diag[i] = 1 / vals64[diag_slot[i]] (ngs_finish_system without the FP32 copy of the values) */
 int ngs_csr_inv_diag(const double* vals64, const int64_t* diag_slot, int64_t n, float* inv_diag, ngs_stream s);
+/* The same for any CSR: the entries of row i with column i are summed (none: 1 / 0). */
+int ngs_csr_diag_inv(const int64_t* rowptr, const int32_t* cols, const double* vals64, int64_t n, float* inv_diag,
+                     ngs_stream s);
 /* col_delta[j] = cols[j] - row(j) for a CSR whose every |column - row| fits int16 (the caller
  * checks the bound; ref: no counterpart, the reference's SpMV reads int32 columns,
  * csrc/sparse_solve/solve_pcg.cu:67-73). */

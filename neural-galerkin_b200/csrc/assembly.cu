@@ -680,6 +680,34 @@ __global__ void inv_diag_kernel(const double* __restrict__ v64, const int64_t* _
   for (int64_t i = ngs_gtid(); i < n; i += ngs_gstride()) inv_diag[i] = (float)(1.0 / v64[diag_slot[i]]);
 }
 
+// 1 / (sum of a row's entries on the diagonal) of any CSR, eight lanes a row.  As torch operations (row of every
+// entry, mask, two selections with their synchronisations, scatter) this took 0.30 of the 1.72 ms of a direct-solve
+// replacement with 7M entries; bound by the 12 bytes of an entry's column (and the values on the diagonal).
+__global__ void diag_inv_kernel(const int64_t* __restrict__ rp, const int32_t* __restrict__ cols,
+                                const double* __restrict__ vals, int64_t n, float* __restrict__ inv_diag) {
+  const int sub = threadIdx.x & 7;
+  const unsigned mask = 0xffu << (threadIdx.x & 24);
+  for (int64_t row = ngs_gtid() >> 3; row < n; row += ngs_gstride() >> 3) {
+    double d = 0.0;
+    const int64_t end = rp[row + 1];
+#pragma unroll 4
+    for (int64_t j = rp[row] + sub; j < end; j += 8)
+      if (cols[j] == row) d += vals[j];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) d += __shfl_xor_sync(mask, d, o);
+    if (sub == 0) inv_diag[row] = (float)(1.0 / d);
+  }
+}
+
+extern "C" int ngs_csr_diag_inv(const int64_t* rowptr, const int32_t* cols, const double* vals64, int64_t n,
+                                float* inv_diag, ngs_stream s) {
+  if (n < 0 || (n > 0 && (!rowptr || !cols || !vals64 || !inv_diag))) return NGS_ERR_INVALID_ARG;
+  if (n == 0) return NGS_OK;
+  { ngs_count_launch(); diag_inv_kernel<<<ngs_blocks(n * 8, 256), 256, 0, (cudaStream_t)s>>>(rowptr, cols, vals64, n, inv_diag); }
+  NGS_CHECK_LAUNCH();
+  return NGS_OK;
+}
+
 extern "C" int ngs_csr_inv_diag(const double* vals64, const int64_t* diag_slot, int64_t n, float* inv_diag,
                                 ngs_stream s) {
   if (n < 0 || (n > 0 && (!vals64 || !diag_slot || !inv_diag))) return NGS_ERR_INVALID_ARG;

@@ -151,6 +151,7 @@ _SIGS = {
     "ngs_pcg_pack_col_words": ([i64, i64, C.c_int], i64),
     "ngs_pcg_pack_count": ([vp, i64, vp, vp], C.c_int),
     "ngs_pcg_pack_fill": ([vp, vp, vp, i64, vp, C.c_int, C.c_int, vp, vp, vp], C.c_int),
+    "ngs_csr_diag_inv": ([vp, vp, vp, i64, vp, vp], C.c_int),
     "ngs_csr_inv_diag": ([vp, vp, i64, vp, vp], C.c_int),
     "ngs_csr_col_delta": ([vp, vp, i64, vp, vp], C.c_int),
     "ngs_mf_count": ([vp, i64, i64, vp, vp, vp], C.c_int),

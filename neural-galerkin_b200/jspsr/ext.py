@@ -209,12 +209,17 @@ def solve_cusparse(Ap, Aj, Ax, b, tol: float):
     """Direct-solve replacement (``solve_cusparse.cu:15-42``): FP64 PCG to 1e-12 relative residual."""
     _check_cuda(Ap, Aj, Ax, b)
     n = b.shape[0]
-    rowptr = Ap.long()
-    rows = torch.repeat_interleave(torch.arange(n, device=b.device), rowptr[1:] - rowptr[:-1])
-    ax64 = Ax.double()
-    diag = torch.zeros(n, dtype=torch.float64, device=b.device).index_add_(0, rows[Aj.long() == rows],
-                                                                            ax64[Aj.long() == rows])
-    x, _ = _pcg(Ap, Aj, Ax, b, (1.0 / diag).float(), 1e-12, -1, False, L.PCG_FP64, b64=b.double(), ax64=ax64)
+    rowptr, cols, ax64 = Ap.contiguous().long(), Aj.contiguous().int(), Ax.contiguous().double()
+    if rowptr.shape != (n + 1,) or cols.numel() != ax64.numel():
+        raise ValueError(f"CSR of {rowptr.numel() - 1} rows, {cols.numel()} columns and {ax64.numel()} values for {n} unknowns")
+    if n > 0:
+        counts = rowptr[1:] - rowptr[:-1]
+        total, least = torch.stack([counts.sum(), counts.min()]).tolist()
+        if total != cols.numel() or least < 0:
+            raise ValueError(f"row pointers of {total} entries (smallest row {least}) for {cols.numel()} columns")
+    inv_diag = torch.empty(n, dtype=torch.float32, device=b.device)
+    L.call("ngs_csr_diag_inv", L.ptr(rowptr), L.ptr(cols), L.ptr(ax64), n, L.ptr(inv_diag), L.stream())
+    x, _ = _pcg(rowptr, cols, Ax, b, inv_diag, 1e-12, -1, False, L.PCG_FP64, b64=b.double(), ax64=ax64)
     return x
 
 
