@@ -497,8 +497,10 @@ def main():
     lv0 = rec.levels[0]
     pcg_ms = {d: rec.pcg_ms[d] for d in rec.pcg_ms}
     iters0 = stats[0]["iters"]
-    # algorithmic bytes per PCG iteration: 8 B per non-zero (FP32 value + int32 column) + 48 B per row
-    alg_bytes = iters0 * (8 * lv0.nnz + 48 * lv0.n)
+    # algorithmic bytes per PCG iteration: 6 B per non-zero (FP32 value + 2-byte column; 8 where the deltas do not
+    # fit 2 bytes) + 48 B per row
+    per_nnz = 8 if lv0.pk_vals is None or rec.pk_wide(lv0) else 6
+    alg_bytes = iters0 * (per_nnz * lv0.nnz + 48 * lv0.n)
     achieved = alg_bytes / (pcg_ms[0] / 1e3) / 1e9
     peaks = {}
     pk = ROOT / "MEASURED_PEAKS.json"

@@ -54,11 +54,14 @@ class AdditiveTerms:
     def of(basis, shapes, feats_list, normals_list):
         """The terms for these shapes, or None where a tensor or the basis needs the torch form."""
         from .additive import AdditiveBasis
+        from .hermite_ns import AdditiveHermite
         cls = type(basis)
         if not issubclass(cls, AdditiveBasis) or torch.are_deterministic_algorithms_enabled():
             return None
         if any(getattr(cls, m) is not getattr(AdditiveBasis, m) for m in
                ("evaluate", "integrate_deriv_deriv_product", "integrate_const_deriv_product", "_buf")):
+            return None
+        if cls.feature_to_coefficient not in (AdditiveBasis.feature_to_coefficient, AdditiveHermite.feature_to_coefficient):
             return None
         comps = component_table(basis.components)
         if comps is None:

@@ -62,8 +62,8 @@ def footprint_bytes(n_points: int, voxel_size: float, depth: int = 4) -> int:
     """Estimated peak device memory of one reconstruction.
 
     Per point: inputs, density / level / weight and the 27-entry basis rows of every level
-    (about 0.25 KB per level).  Per voxel: the CSR row of up to 125 entries in FP64 + FP32 + int32
-    (2 KB), solve vectors and mesh buffers.  The voxel count of a level is bounded by the points'
+    (about 0.25 KB per level).  Per voxel: the CSR row (about 60 of up to 125 entries) in FP64 + int32
+    and the solver's packed copy of it (1.3 of the 2 KB), solve vectors and mesh buffers.  The voxel count of a level is bounded by the points'
     trilinear corners (8 per point) and by the surface the cloud can span at that voxel size.
     """
     per_point = 96 + 256 * depth
