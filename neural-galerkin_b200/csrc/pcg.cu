@@ -11,8 +11,8 @@
 //     barrier + reduce     every block publishes its partials, arrives, and once all
 //                          have arrived sums all partials itself in block order
 //                          (deterministic, the same bits in every block).
-// The SpMV streams the CSR arrays straight from HBM: eight lanes per row at two blocks per SM,
-// in one of two forms -- 4-byte columns, a row at a time with up to eight (column, value) pairs
+// The SpMV streams the matrix straight from HBM, eight lanes per row at two blocks per SM: a packed
+// copy of it (four rows to a warp, at spmv_packed), or a caller's CSR in one of two forms -- 4-byte columns, a row at a time with up to eight (column, value) pairs
 // and their vector gathers in flight per lane, or 2-byte column deltas in a software-pipelined
 // loop that gathers from a shared-memory window of the vector -- each with its own kernel for the
 // single-system and cluster solves.  (Staging CSR tiles through shared memory with bulk copies ran
