@@ -50,7 +50,7 @@ class EvalFunc(torch.autograd.Function):
         table = axes_table(components, xyz, coeffs, feat_ids)
         with torch.no_grad():
             if table is not None:
-                out = torch.empty(xyz.shape, device=xyz.device)
+                out = torch.empty(xyz.shape, dtype=torch.float32, device=xyz.device)
                 for k in range(0, xyz.shape[0], AXES_CHUNK):
                     rows, x = coeffs[feat_ids[k:k + AXES_CHUNK]], xyz[k:k + AXES_CHUNK].contiguous()
                     L.call("ngs_basis_axes", C.byref(table), L.ptr(rows), L.ptr(x), x.shape[0], L.ptr(out[k:]), L.stream())
@@ -68,10 +68,10 @@ class EvalFunc(torch.autograd.Function):
         xyz, ids = ctx.saved_tensors
         with torch.no_grad():
             if ctx.table is not None and grad.dtype == torch.float32:
-                out = torch.zeros((ctx.n, 3 * len(ctx.components)), device=xyz.device)
+                out = torch.zeros((ctx.n, 3 * len(ctx.components)), dtype=torch.float32, device=xyz.device)
                 for k in range(0, xyz.shape[0], AXES_CHUNK):
                     x, gk = xyz[k:k + AXES_CHUNK].contiguous(), grad[k:k + AXES_CHUNK].contiguous()
-                    g = torch.empty((x.shape[0], out.shape[1]), device=x.device)
+                    g = torch.empty((x.shape[0], out.shape[1]), dtype=torch.float32, device=x.device)
                     L.call("ngs_basis_axes_grad", C.byref(ctx.table), L.ptr(x), L.ptr(gk), x.shape[0], L.ptr(g), L.stream())
                     out.index_add_(0, ids[k:k + AXES_CHUNK], g)
                 return None, out, None, None
