@@ -376,11 +376,16 @@ NGS_DEV void spmv_packed(const PcgArgs& a, const VT* v, int64_t row0, int64_t ro
 // The streaming choice is a template argument: one load form per instantiation (a runtime choice
 // per load cost 7 % of the level-0 solve and forced register spills).  FORM picks the SpMV form at
 // compile time (kernels specialised per form, so that one form's register allocation is not shaped
-// by the others') or, with PCG_FORM_ANY, at run time from the system (one kernel for every system of
-// a batch or a cluster launch).  Each form runs the same uncontracted arithmetic in every kernel, so
-// a system's result does not depend on which kernel solved it.
+// by the others') or at run time from the system: among the caller's CSR forms (PCG_FORM_ANY) or among the
+// packed ones (PCG_FORM_PACKED_ANY); all of them together (PCG_FORM_ALL) only in a batch that mixes both, where
+// registers spill (FP64 mode: 148 bytes of stores and 272 of loads against none for the CSR forms).  One kernel with
+// all of them for every system took, against a kernel per kind: reference mode, alone, 180,000 rows, 1.80 ms against
+// 1.05; a batched launch of the mixed mode 2.22 against 1.56.  Each form runs the same uncontracted arithmetic in
+// every kernel, so a system's result does not depend on which kernel solved it.
 constexpr int PCG_FORM_ANY = 0, PCG_FORM_DELTA_STREAM = 1, PCG_FORM_DELTA = 2, PCG_FORM_COLS_STREAM = 3,
-              PCG_FORM_COLS = 4, PCG_FORM_PACKED = 5;      // 5 .. 8: + 1 streamed, + 2 4-byte columns
+              PCG_FORM_COLS = 4, PCG_FORM_PACKED = 5,      // 5 .. 8: + 1 streamed, + 2 4-byte columns
+              PCG_FORM_PACKED_ANY = 9,                     // 5 .. 8 at run time
+              PCG_FORM_ALL = 10;                           // CSR and packed at run time
 
 template <int FORM, typename MT, typename VT, typename ACC, typename Pre, typename Epi>
 NGS_DEV void spmv_rows(const PcgArgs& a, const MT* __restrict__ vals, const VT* v, int64_t voff, int64_t row0,
@@ -391,7 +396,7 @@ NGS_DEV void spmv_rows(const PcgArgs& a, const MT* __restrict__ vals, const VT* 
     spmv_rows_piped<false, true, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
   } else if constexpr (FORM == PCG_FORM_COLS_STREAM) {
     spmv_rows_plain<true, false, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
-  } else if constexpr (FORM == PCG_FORM_COLS || FORM >= PCG_FORM_PACKED) {   // packed: the true residual's
+  } else if constexpr (FORM == PCG_FORM_COLS || (FORM >= PCG_FORM_PACKED && FORM != PCG_FORM_ALL)) {   // packed: the true residual's
     spmv_rows_plain<false, false, MT, VT, ACC>(a, vals, v, voff, row0, row1, pre, epi, dsum);
   } else if (a.cols16) {
     // the column encoding too: 2-byte deltas when the caller supplied them, 4-byte columns otherwise
@@ -698,11 +703,14 @@ NGS_DEV void pcg_body(const PcgArgs& a, const unsigned bid, Sync& sy) {
     if (!a.mf && rows_ok && a.win_cap > 0) csr_window(a, row0, row1, win_bounds[0], win_bounds[1]);
   }
   auto spmv_w = [&](double& sum) {
-    if constexpr (FORM >= PCG_FORM_PACKED) {
+    if constexpr (FORM == PCG_FORM_PACKED_ANY) {
+      spmv_packed_any<MT, VT, ACC>(a, u, row0, row1, w_pre, w_epi, sum);
+      return;
+    } else if constexpr (FORM >= PCG_FORM_PACKED && FORM < PCG_FORM_PACKED_ANY) {
       constexpr int F = FORM - PCG_FORM_PACKED;
       spmv_packed<(F & 1) != 0, (F & 2) != 0, MT, VT, ACC>(a, u, row0, row1, w_pre, w_epi, sum);
       return;
-    } else if constexpr (FORM == PCG_FORM_ANY) {
+    } else if constexpr (FORM == PCG_FORM_ALL) {
       if (a.pk_start) {
         spmv_packed_any<MT, VT, ACC>(a, u, row0, row1, w_pre, w_epi, sum);
         return;
@@ -858,7 +866,7 @@ NGS_DEV void pcg_body(const PcgArgs& a, const unsigned bid, Sync& sy) {
       replacements++;
       for (int64_t i = i0; i < i1; i += is) part[0] += (double)r[i] * (double)u[i];
       if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
-      const double rec = rho;
+      const bool drifted = res[2] > PCG_DRIFT * rho;
       gamma_new = res[0];
       rho = res[2];
       if (sqrt(rho) <= atol) { converged = true; break; }
@@ -870,7 +878,7 @@ NGS_DEV void pcg_body(const PcgArgs& a, const unsigned bid, Sync& sy) {
       // The search directions go on from the replaced residual; only where the recurrence had drifted far from
       // it do they start anew.  (Starting anew at every refinement lost the directions that the conjugate
       // gradients had found: 54 iterations instead of 52 on level 0 of a 300k-point cloud.)
-      if (rho > PCG_DRIFT * rec) {
+      if (drifted) {
         gamma = gamma_new;
         alpha = delta != 0.0 ? gamma / delta : 0.0;
         beta = 0.0;
@@ -935,7 +943,7 @@ struct PcgBatch {
 };
 static_assert(sizeof(PcgBatch) <= 32000, "batch arguments must fit the kernel parameter space");
 
-template <int MODE, int OPS>
+template <int MODE, int OPS, int FORM = PCG_FORM_ANY>
 __global__ void __launch_bounds__(PCG_THREADS, PCG_MIN_BLOCKS) pcg_batch_kernel(const __grid_constant__ PcgBatch b) {
   int lo = 0, hi = b.nsys - 1;              // last system whose first block is <= blockIdx.x
   while (lo < hi) {
@@ -943,7 +951,7 @@ __global__ void __launch_bounds__(PCG_THREADS, PCG_MIN_BLOCKS) pcg_batch_kernel(
     if (b.start[mid] <= blockIdx.x) lo = mid; else hi = mid - 1;
   }
   GridSync sy(b.sys[lo], blockIdx.x - b.start[lo]);
-  pcg_body<MODE, OPS, PCG_FORM_ANY>(b.sys[lo], blockIdx.x - b.start[lo], sy);
+  pcg_body<MODE, OPS, FORM>(b.sys[lo], blockIdx.x - b.start[lo], sy);
 }
 
 // Small systems of a batch that have one cluster size and one SpMV form: a cluster each, in one launch.  A system's
@@ -1021,6 +1029,10 @@ static int pcg_capacity() {
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_kernel<MODE, PCG_OPS_MF>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_MF>));
     per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_BOTH>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_CSR, PCG_FORM_PACKED>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_CSR, PCG_FORM_PACKED_ANY>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_CSR, PCG_FORM_ALL>));
+    per_sm = std::min(per_sm, pcg_occupancy((const void*)pcg_batch_kernel<MODE, PCG_OPS_BOTH, PCG_FORM_ALL>));
   }
   const int64_t cap = (int64_t)sms * per_sm;
   const int out = (int)(cap < PCG_MAX_BLOCKS ? cap : PCG_MAX_BLOCKS);   // the partials area holds this many
@@ -1084,6 +1096,7 @@ static int pcg_cluster_limit() {
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_DELTA>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_COLS>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED>));
+    limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED_ANY>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_DELTA>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_COLS>));
     limit = std::min(limit, pcg_cluster_limit_of_kernel((const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_PACKED>));
@@ -1177,6 +1190,7 @@ struct PcgClusterKernels {
 
 template <int MODE>
 static PcgClusterKernels pcg_cluster_forms(const PcgArgs& a) {
+  if (a.pk_start && (a.pk_wide || a.evict_first)) return {(const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED_ANY>, nullptr};
   if (a.pk_start) return {(const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_PACKED>,
                           (const void*)pcg_cluster_batch_kernel<MODE, PCG_FORM_PACKED>};
   if (a.cols16) return {(const void*)pcg_cluster_form_kernel<MODE, PCG_FORM_DELTA>,
@@ -1186,7 +1200,7 @@ static PcgClusterKernels pcg_cluster_forms(const PcgArgs& a) {
 }
 
 static PcgClusterKernels pcg_cluster_kernels_of(const PcgArgs& a, int mode) {
-  if (mode == NGS_PCG_REFERENCE || a.mf || a.evict_first || (a.pk_start && a.pk_wide))
+  if (mode == NGS_PCG_REFERENCE || a.mf || (a.evict_first && !a.pk_start))
     return {pcg_cluster_kernel_of(mode, a.mf != 0), nullptr};
   return mode == NGS_PCG_MIXED ? pcg_cluster_forms<NGS_PCG_MIXED>(a) : pcg_cluster_forms<NGS_PCG_FP64>(a);
 }
@@ -1329,22 +1343,45 @@ static void* pcg_kernel_of(int mode, bool mf) {
   return mf ? (void*)pcg_kernel<NGS_PCG_FP64, PCG_OPS_MF> : (void*)pcg_kernel<NGS_PCG_FP64, PCG_OPS_CSR>;
 }
 
-// ops: PCG_OPS_CSR / _MF / _BOTH, from the systems of the batch.
+// The kernel of a batch's cooperative launch, by the kinds of its systems: the one that carries no more forms than
+// they need.
+struct PcgBatchKinds {
+  bool csr, mf, packed, other;              // other: packed with 4-byte columns or streamed
+};
+
 template <int MODE>
-static void* pcg_batch_kernel_ops(int ops) {
+static void* pcg_batch_kernel_for(const PcgBatchKinds& k) {
   if constexpr (MODE == NGS_PCG_REFERENCE) {
     return (void*)pcg_batch_kernel<MODE, PCG_OPS_CSR>;
   } else {
-    if (ops == PCG_OPS_MF) return (void*)pcg_batch_kernel<MODE, PCG_OPS_MF>;
-    if (ops == PCG_OPS_BOTH) return (void*)pcg_batch_kernel<MODE, PCG_OPS_BOTH>;
-    return (void*)pcg_batch_kernel<MODE, PCG_OPS_CSR>;
+    if (!k.packed && !k.other) {
+      if (!k.mf) return (void*)pcg_batch_kernel<MODE, PCG_OPS_CSR>;
+      return k.csr ? (void*)pcg_batch_kernel<MODE, PCG_OPS_BOTH> : (void*)pcg_batch_kernel<MODE, PCG_OPS_MF>;
+    }
+    if (k.mf) return (void*)pcg_batch_kernel<MODE, PCG_OPS_BOTH, PCG_FORM_ALL>;
+    if (k.csr) return (void*)pcg_batch_kernel<MODE, PCG_OPS_CSR, PCG_FORM_ALL>;
+    return k.other ? (void*)pcg_batch_kernel<MODE, PCG_OPS_CSR, PCG_FORM_PACKED_ANY>
+                   : (void*)pcg_batch_kernel<MODE, PCG_OPS_CSR, PCG_FORM_PACKED>;
   }
 }
 
-static void* pcg_batch_kernel_of(int mode, int ops) {
-  if (mode == NGS_PCG_REFERENCE) return pcg_batch_kernel_ops<NGS_PCG_REFERENCE>(ops);
-  if (mode == NGS_PCG_MIXED) return pcg_batch_kernel_ops<NGS_PCG_MIXED>(ops);
-  return pcg_batch_kernel_ops<NGS_PCG_FP64>(ops);
+static void* pcg_batch_kernel_of(int mode, const PcgBatchKinds& k) {
+  if (mode == NGS_PCG_REFERENCE) return pcg_batch_kernel_for<NGS_PCG_REFERENCE>(k);
+  if (mode == NGS_PCG_MIXED) return pcg_batch_kernel_for<NGS_PCG_MIXED>(k);
+  return pcg_batch_kernel_for<NGS_PCG_FP64>(k);
+}
+
+// The blocks of one system, alone in a cooperative launch.
+static int launch_solo(PcgArgs& a, int mode, cudaStream_t st) {
+  cudaMemsetAsync(a.count, 0, 8 * sizeof(unsigned int), st);
+  void* args[] = {&a};
+  ngs_count_launch();
+  void* f = a.mf ? pcg_kernel_of(mode, true)
+            : mode == NGS_PCG_MIXED ? pcg_form_kernel_for<NGS_PCG_MIXED>(a)
+            : mode == NGS_PCG_FP64 ? pcg_form_kernel_for<NGS_PCG_FP64>(a)
+            : pcg_kernel_of(mode, false);
+  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(a.nblocks), dim3(PCG_THREADS), args, pcg_win_smem(a), st);
+  return e == cudaSuccess ? NGS_OK : ngs_set_cuda_error(e);
 }
 
 extern "C" int ngs_pcg_solve(const ngs_pcg_system* sys, const ngs_pcg_config* cfg, void* ws, size_t ws_bytes,
@@ -1366,17 +1403,7 @@ extern "C" int ngs_pcg_solve(const ngs_pcg_system* sys, const ngs_pcg_config* cf
   if (blocks < 1) return NGS_ERR_INVALID_ARG;
   a.nblocks = (unsigned int)blocks;
   pcg_set_window(a, cfg->mode, sys->band, blocks);
-  cudaMemsetAsync(a.count, 0, 8 * sizeof(unsigned int), st);
-  void* args[] = {&a};
-  ngs_count_launch();
-  void* f = a.mf ? pcg_kernel_of(cfg->mode, true)
-             : cfg->mode == NGS_PCG_MIXED ? pcg_form_kernel_for<NGS_PCG_MIXED>(a)
-             : cfg->mode == NGS_PCG_FP64 ? pcg_form_kernel_for<NGS_PCG_FP64>(a)
-             : pcg_kernel_of(cfg->mode, false);
-  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3((unsigned)blocks), dim3(PCG_THREADS), args, pcg_win_smem(a),
-                                                    st);
-  if (e != cudaSuccess) return ngs_set_cuda_error(e);
-  return NGS_OK;
+  return launch_solo(a, cfg->mode, st);
 }
 
 extern "C" int ngs_pcg_solve_batch(const ngs_pcg_batch_item* items, int n_items, ngs_stream s) {
@@ -1453,20 +1480,20 @@ extern "C" int ngs_pcg_solve_batch(const ngs_pcg_batch_item* items, int n_items,
   }
   if (b.nsys == 0) return NGS_OK;
   b.start[b.nsys] = total;
-  for (int k = 0; k < b.nsys; k++) {
-    pcg_clear_status(b.sys[k].info, b.sys[k].resid, st);
-    cudaMemsetAsync(b.sys[k].count, 0, 8 * sizeof(unsigned int), st);
-  }
-  int ops = 0;
+  PcgBatchKinds kinds{};
   size_t smem = 0;
   for (int k = 0; k < b.nsys; k++) {
-    ops |= b.sys[k].mf ? PCG_OPS_MF : PCG_OPS_CSR;
-    smem = std::max(smem, pcg_win_smem(b.sys[k]));
+    const PcgArgs& a = b.sys[k];
+    pcg_clear_status(a.info, a.resid, st);
+    (a.mf ? kinds.mf : !a.pk_start ? kinds.csr : a.pk_wide || a.evict_first ? kinds.other : kinds.packed) = true;
+    smem = std::max(smem, pcg_win_smem(a));
   }
+  if (b.nsys == 1) return launch_solo(b.sys[0], mode, st);
+  for (int k = 0; k < b.nsys; k++) cudaMemsetAsync(b.sys[k].count, 0, 8 * sizeof(unsigned int), st);
   void* args[] = {&b};
   ngs_count_launch();
-  void* f = pcg_batch_kernel_of(mode, ops);
-  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(total), dim3(PCG_THREADS), args, smem, st);
+  const cudaError_t e = cudaLaunchCooperativeKernel(pcg_batch_kernel_of(mode, kinds), dim3(total), dim3(PCG_THREADS), args,
+                                                    smem, st);
   if (e != cudaSuccess) return ngs_set_cuda_error(e);
   return NGS_OK;
 }
