@@ -111,6 +111,7 @@ class Level:
     pk_units: int = 0                # units in all, values and columns
     pk_vals: torch.Tensor = None
     pk_cols: torch.Tensor = None
+    pk_mode: int = None              # the solver mode its values are stored for
     # matrix-free operator (solver reads no CSR): the point basis transposed per row
     group: tuple = None            # (sorted cell keys, point order): screening terms of long-pair levels
     pair_form: bool = False        # screening terms gathered per row from the transposed pairs
@@ -593,6 +594,7 @@ class Reconstruction(DualMesher):
                                      device=self.dev)
             L.call("ngs_pcg_pack_fill", L.ptr(lv.rowptr), L.ptr(lv.cols), L.ptr(lv.vals64), lv.n, L.ptr(lv.pk_start), wide,
                    mode, L.ptr(lv.pk_vals), L.ptr(lv.pk_cols), st)
+            lv.pk_mode = mode
             L.call("ngs_csr_inv_diag", L.ptr(lv.vals64), L.ptr(lv.diag_slot), lv.n, L.ptr(inv_diag), st)
         else:
             lv.vals32_ = torch.empty(lv.nnz, dtype=torch.float32, device=self.dev)
@@ -705,11 +707,12 @@ class Reconstruction(DualMesher):
             sysd.nnz = lv.nnz
             sysd.rowptr, sysd.cols = lv.rowptr.data_ptr(), lv.cols.data_ptr()
             sysd.vals64 = lv.vals64.data_ptr()
-            if lv.pk_vals is not None:
+            if lv.pk_vals is not None and lv.pk_mode == spec.mode:
                 sysd.pk_start, sysd.pk_vals, sysd.pk_cols = (t.data_ptr() for t in (lv.pk_start, lv.pk_vals, lv.pk_cols))
                 sysd.pk_units, sysd.pk_wide = lv.pk_units, self.pk_wide(lv)
                 b32 = None
             else:
+                # also where the solver was changed after the assembly: the packed values are of another mode's type
                 sysd.vals32, sysd.band = lv.vals32.data_ptr(), lv.band
                 b32 = lv.rhs.float()
                 sysd.b32 = b32.data_ptr()
