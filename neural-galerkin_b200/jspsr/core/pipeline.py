@@ -112,6 +112,7 @@ class Level:
     pk_vals: torch.Tensor = None
     pk_cols: torch.Tensor = None
     pk_mode: int = None              # the solver mode its values are stored for
+    col_delta: torch.Tensor = None   # int16 column - row per non-zero, for levels solved from the CSR
     # matrix-free operator (solver reads no CSR): the point basis transposed per row
     group: tuple = None            # (sorted cell keys, point order): screening terms of long-pair levels
     pair_form: bool = False        # screening terms gathered per row from the transposed pairs
@@ -585,7 +586,7 @@ class Reconstruction(DualMesher):
             L.call("ngs_screen_gram_grouped", L.ptr(lv.rows), L.ptr(lv.phi), self.n, None, L.ptr(order),
                    L.ptr(keys), L.ptr(lv.masks), L.ptr(lv.rowptr), self._screen_scale(d), L.ptr(lv.vals64), st)
         inv_diag = torch.empty(lv.n, dtype=torch.float32, device=self.dev)
-        if lv.pk_start is not None and not lv.mf:
+        if self._packs(lv):
             # the solver's copy: values in its precision, 2-byte column deltas where every |column - row| fits
             mode, wide = self.solver.mode, self.pk_wide(lv)
             lv.pk_vals = torch.empty(lv.pk_units * 32, dtype=torch.float32 if mode == L.PCG_MIXED else torch.float64,
@@ -597,11 +598,29 @@ class Reconstruction(DualMesher):
             lv.pk_mode = mode
             L.call("ngs_csr_inv_diag", L.ptr(lv.vals64), L.ptr(lv.diag_slot), lv.n, L.ptr(inv_diag), st)
         else:
+            mode = self.solver.mode
+            if (not lv.mf and mode is not None and lv.band <= 32767 and
+                    L.load().ngs_pcg_window(lv.n, lv.nnz, lv.band, mode) == 1):
+                # 2-byte column deltas where every |column - row| fits and the solver reads them (the launches
+                # that stage the vector in shared memory): 6 instead of 8 bytes per non-zero
+                lv.col_delta = torch.empty(lv.nnz, dtype=torch.int16, device=self.dev)
+                L.call("ngs_csr_col_delta", L.ptr(lv.rowptr), L.ptr(lv.cols), lv.n, L.ptr(lv.col_delta), st)
             lv.vals32_ = torch.empty(lv.nnz, dtype=torch.float32, device=self.dev)
             L.call("ngs_finish_system", L.ptr(lv.vals64), lv.nnz, L.ptr(lv.diag_slot), lv.n, L.ptr(lv.vals32_),
                    L.ptr(inv_diag), st)
         if not lv.mf:
             lv.inv_diag = inv_diag
+
+    def _packs(self, lv: Level) -> bool:
+        """Whether the solver gets a packed copy of the level's matrix (mixed and FP64 modes), or reads the CSR.
+
+        The packed form pads four rows to the longest of them and to a multiple of eight entries: short rows
+        lose by it.  Time of a product, packed over CSR, by the mean entries of a row (mixed / FP64): 11 entries
+        1.28 / 1.19, 14: 1.26 / 1.23, 20: 1.15 / 1.14, 32: 1.12 / 1.12, 33: 1.01 / 1.00, 48: 0.98 / 0.93,
+        60 and more: 0.82 to 0.99.  Small systems of the mixed mode have their vector in shared memory with the CSR:
+        4,387 rows 1.05, 5,333 rows 1.06, 11,500 rows 0.96 (FP64: 0.83, 0.81, 0.83)."""
+        return (lv.pk_start is not None and not lv.mf and lv.nnz >= 40 * lv.n and
+                (self.solver.mode == L.PCG_FP64 or lv.n >= 8192))
 
     @staticmethod
     def pk_wide(lv: Level) -> int:
@@ -714,6 +733,7 @@ class Reconstruction(DualMesher):
             else:
                 # also where the solver was changed after the assembly: the packed values are of another mode's type
                 sysd.vals32, sysd.band = lv.vals32.data_ptr(), lv.band
+                sysd.col_delta = lv.col_delta.data_ptr() if lv.col_delta is not None else None
                 b32 = lv.rhs.float()
                 sysd.b32 = b32.data_ptr()
         sysd.b64 = lv.rhs.data_ptr()
