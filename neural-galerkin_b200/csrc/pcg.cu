@@ -48,7 +48,6 @@ constexpr int PCG_ROW_LANES = 8;       // lanes per row in the SpMV
 constexpr int PCG_GROUP_ROWS = 4;      // rows of a group of the packed form: a warp's, eight lanes each
 constexpr int PCG_ROW_COST = 8;        // work of a row on top of its non-zeros (vector traffic)
 constexpr int PCG_BLOCK_WORK = 16384;  // work (non-zeros + row cost) that justifies one more block
-constexpr double PCG_DRIFT = 16.0;     // true over recurrence residual (squared) that restarts the directions
 constexpr int PCG_CLUSTER_MAX = 16;    // CTAs of the largest thread-block cluster a small system gets
 constexpr int PCG_CLUSTER_NEED = 64;   // systems of at most this many blocks' work are solved by a cluster
 // Most blocks one cooperative solve may use (B200: 148 SMs x 2 = 296).  The capacity query clamps to
@@ -854,36 +853,31 @@ NGS_DEV void pcg_body(const PcgArgs& a, const unsigned bid, Sync& sy) {
     if (!apply_w(part[1])) return pcg_abandon(a, it);
     if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
     it++;
-    double gamma_new = res[0];
+    const double gamma_new = res[0];
     delta = res[1];
     rho = res[2];
     if (sqrt(rho) <= target) {
       if (MODE != NGS_PCG_MIXED) { converged = true; break; }
-      // the recurrence residual is down: the true FP64 residual takes its place
+      // end of an inner solve: true FP64 residual, stop or restart the recurrences from it.  (Going on with the old
+      // search directions, 52 instead of 54 iterations on level 0 of a 300k-point cloud, loses convergence: the
+      // 7-point Laplacian of 40^3 rows, shifted by 1e-4, takes 406 iterations to 1e-7, and with the old directions
+      // stays at 4e-4 until the iteration cap.)
       if (!sy.barrier()) return pcg_abandon(a, it);
       part[0] = part[1] = part[2] = 0.0;
       if (!apply_true(part[2])) return pcg_abandon(a, it);
       replacements++;
       for (int64_t i = i0; i < i1; i += is) part[0] += (double)r[i] * (double)u[i];
-      if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
-      const bool drifted = res[2] > PCG_DRIFT * rho;
-      gamma_new = res[0];
-      rho = res[2];
-      if (sqrt(rho) <= atol) { converged = true; break; }
-      part[0] = part[1] = part[2] = 0.0;
+      if (!sy.barrier()) return pcg_abandon(a, it);
       if (!apply_w(part[1])) return pcg_abandon(a, it);
       if (!sy.template reduce<3>(part, res)) return pcg_abandon(a, it);
+      rho = res[2];
+      if (sqrt(rho) <= atol) { converged = true; break; }
+      gamma = res[0];
       delta = res[1];
+      alpha = delta != 0.0 ? gamma / delta : 0.0;
+      beta = 0.0;
       target = fmax(atol, rtol_inner * sqrt(rho));
-      // The search directions go on from the replaced residual; only where the recurrence had drifted far from
-      // it do they start anew.  (Starting anew at every refinement lost the directions that the conjugate
-      // gradients had found: 54 iterations instead of 52 on level 0 of a 300k-point cloud.)
-      if (drifted) {
-        gamma = gamma_new;
-        alpha = delta != 0.0 ? gamma / delta : 0.0;
-        beta = 0.0;
-        continue;
-      }
+      continue;
     }
     beta = gamma != 0.0 ? gamma_new / gamma : 0.0;
     const double den = delta - beta * gamma_new / alpha;
