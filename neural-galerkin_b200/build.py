@@ -39,7 +39,7 @@ def nvcc() -> str:
 
 
 def _newest_dep() -> float:
-    deps = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.inc")) + list(INCLUDE.glob("*.h"))
+    deps = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(CSRC.glob("*.inc")) + list(INCLUDE.glob("*.h"))
     return max(p.stat().st_mtime for p in deps)
 
 

@@ -24,6 +24,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include "conv_ring.h"
 #include "ngs_common.cuh"
 
 namespace conv {
@@ -328,11 +329,16 @@ NGS_DEV void run_tile(const TileShape& t, uint8_t* smem, Fill& fill, Store& stor
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_flag) {
+    int late = 0;                                // the MMAs issued end before their tensor memory is given up
+    if (warp == PRODUCERS / 32 && lane == 0) mbar_wait(&done_bar, 0u, &late);
+    if (tid == 0) atomicExch(error, NGS_ERR_TIMEOUT);
+    __syncwarp();
+  }
   if (warp == PRODUCERS / 32) {
     tc_fence_after();
     tmem_free(tmem, ncols_alloc);
   }
-  if (tid == 0 && abort_flag) atomicExch(error, NGS_ERR_TIMEOUT);
 }
 
 NGS_DEV uint4 ldg16(const uint16_t* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
@@ -430,35 +436,24 @@ NGS_DEV void run_tile_tma(const TmaShape& t, uint8_t* smem, Setup& setup, Next& 
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
 
+  RingSpan open{0, 0};                           // steps whose TMA copies may still be on their way
   if (warp == 0 || warp == 6) {
     const int w = warp == 6;
-    int st = 0, s = 0;
-    uint32_t parity = 1u;                        // of the round before this one
-    bool more = true;
-    while (more) {
-      const int valid = next();
-      more = valid > 0;
-      const bool go = s < S || mbar_wait(&empty_bar[st], parity, &abort_flag);
-      if (!__all_sync(0xffffffffu, go)) break;
-      if (lane == 0) {
-        if (w == 0) ksteps_of[st] = (valid + UK - 1) / UK;   // 0: no more steps
-        if (more && t.tx[w] > 0) mbar_expect(&full_bar[st], t.tx[w]);
-        else mbar_arrive(&full_bar[st]);
-      }
-      __syncwarp();
-      if (more) issue(smem + (size_t)st * t.stage_bytes, &full_bar[st], w);
-      s++;
-      if (++st == S) {
-        st = 0;
-        parity ^= 1u;
-      }
-    }
-    // after an abort the copies still land before the shared memory is given up (waits bounded again)
-    if (more && lane == 0)
-      for (int r = max(0, s - S); r < s; r++) {
-        int never = 0;
-        mbar_wait(&full_bar[r % S], (uint32_t)(r / S) & 1u, &never);
-      }
+    open = ring_walk(
+        S, next,
+        [&](int st, uint32_t parity, bool first) {
+          const bool go = first || mbar_wait(&empty_bar[st], parity, &abort_flag);
+          return __all_sync(0xffffffffu, go) != 0;
+        },
+        [&](int st, int valid) {
+          if (lane == 0) {
+            if (w == 0) ksteps_of[st] = (valid + UK - 1) / UK;   // 0: no more steps
+            if (valid > 0 && t.tx[w] > 0) mbar_expect(&full_bar[st], t.tx[w]);
+            else mbar_arrive(&full_bar[st]);
+          }
+          __syncwarp();
+          if (valid > 0) issue(smem + (size_t)st * t.stage_bytes, &full_bar[st], w);
+        });
   } else if (warp >= 2) {
     // a step's copies are handed over while the next one's are in flight (the ring has two stages or more)
     auto hand_over = [&](int st) {
@@ -534,11 +529,20 @@ NGS_DEV void run_tile_tma(const TmaShape& t, uint8_t* smem, Setup& setup, Next& 
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_flag) {
+    // what is in flight ends before the shared and the tensor memory are given up; once one of a thread's waits has
+    // run its full time, the others are not waited for again
+    int late = 0;
+    if ((warp == 0 || warp == 6) && lane == 0)
+      for (int r = open.first; r < open.last; r++) mbar_wait(&full_bar[r % S], (uint32_t)(r / S) & 1u, &late);
+    if (warp == 1 && lane == 0) mbar_wait(&done_bar, 0u, &late);
+    if (tid == 0) atomicExch(error, NGS_ERR_TIMEOUT);
+    __syncwarp();
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_free(tmem, ncols_alloc);
   }
-  if (tid == 0 && abort_flag) atomicExch(error, NGS_ERR_TIMEOUT);
 }
 
 }  // namespace conv
