@@ -642,13 +642,16 @@ extern "C" int ngs_correction_stiffness(const int32_t* fine_coords, int64_t n_fi
                                         const float* x_coarse, const double* tab_c, const double* tab_g, int tab_len,
                                         double* rhs, ngs_stream s) {
   // tables of 3M + 2 entries each: level ratios M up to 2^12 (13 levels) fit one block's shared memory
-  if (n_fine < 0 || fine_stride <= 0 || cg.stride <= fine_stride || tab_len <= 0 || tab_len > 12290)
+  constexpr int MOST = 12290;
+  if (n_fine < 0 || fine_stride <= 0 || cg.stride <= fine_stride || tab_len <= 0 || tab_len > MOST)
     return NGS_ERR_INVALID_ARG;
   if (n_fine == 0) return NGS_OK;
   if (!fine_coords || !cg.words || !x_coarse || !tab_c || !tab_g || !rhs) return NGS_ERR_INVALID_ARG;
   const size_t smem = 2 * (size_t)tab_len * sizeof(double);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(correction_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same limit for every call: another thread's launch may stand between this one's two steps
+    const cudaError_t e = cudaFuncSetAttribute(correction_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               2 * MOST * (int)sizeof(double));
     if (e != cudaSuccess) return ngs_set_cuda_error(e);
   }
   { ngs_count_launch(); correction_kernel<<<ngs_blocks(n_fine, 128), 128, smem, (cudaStream_t)s>>>(

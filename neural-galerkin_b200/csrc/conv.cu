@@ -1086,6 +1086,10 @@ bool rows_map(CUtensorMap& map, const void* base, int64_t width, int64_t rows, i
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Dynamic shared memory of a tile kernel's block, at most (of 227 KB; the static arrays take the rest).  The kernels'
+// limit is always set to this: threads share it, and one with a smaller need would lower it under another's launch.
+constexpr int SMEM_MOST = 226 << 10;
+
 // Stages of the ring for an N-column tile, and the dynamic shared memory of the launch.
 void tile_plan(int n, int& stages, uint32_t& stage_bytes, size_t& smem) {
   const uint32_t nb = (uint32_t)((n + 7) / 8 * 8) * 128u;
@@ -1231,7 +1235,7 @@ static int conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_
     if (g.stages >= 2) break;
   }
   const size_t smem = fixed + (size_t)g.stages * g.stage_bytes;
-  if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
     return ngs_set_cuda_error(cudaGetLastError());
   const dim3 grid((unsigned)((n_rows + conv::BM - 1) / conv::BM), (unsigned)((ncols + 255) / 256));
   ngs_count_launch();
@@ -1300,7 +1304,7 @@ extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const 
   g.error = error_dev;
   size_t smem = 0;
   tile_plan(cout < 256 ? cout : 256, g.stages, g.stage_bytes, smem);
-  if (cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
     return ngs_set_cuda_error(cudaGetLastError());
   const dim3 grid((unsigned)g.splits, (unsigned)K, (unsigned)(g.m_tiles * ((cout + 255) / 256)));
   ngs_count_launch();

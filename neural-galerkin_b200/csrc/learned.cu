@@ -18,6 +18,7 @@
 
 constexpr int BASIS_MOST = 32;        // components of a basis
 constexpr int PAIR_MOST = 12;         // of one whose pair terms run here (registers: three arrays of C floats)
+constexpr int ROWS_SMEM = 4 * 4 * 32 * (3 * BASIS_MOST + 1);   // staged rows of a block of 128 threads, at most
 
 // ----------------------------------------------------------------------------- components
 struct BasisComps {
@@ -306,13 +307,17 @@ __global__ void __launch_bounds__(128) basis_pairs_grad_kernel(const __grid_cons
   }
 }
 
+// Shared memory of a pair kernel's block, at most.  A kernel's limit is set to the most that any call can need, never
+// to a call's own need: threads share it, and one with small tables would lower it under another's launch.
+constexpr int PAIR_SMEM = 200 << 10;
+
 template <int C>
 static int launch_pairs(const PairArgs& a, bool grad, cudaStream_t st) {
   const size_t tab = sizeof(float2) * C * C * a.R;
   const size_t smem = tab + (grad ? sizeof(float) * 4 * 64 * ((3 * C) | 1) : 0);
   const void* f = grad ? (const void*)basis_pairs_grad_kernel<C> : (const void*)basis_pairs_kernel<C>;
   if (smem > 48 << 10) {
-    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
     if (e != cudaSuccess) return ngs_set_cuda_error(e);
   }
   void* args[] = {const_cast<PairArgs*>(&a)};
@@ -324,7 +329,7 @@ static int launch_pairs(const PairArgs& a, bool grad, cudaStream_t st) {
 // Bytes of shared memory of the gradient kernel (the larger of the two) fit a block.
 extern "C" int ngs_basis_pairs_fit(int C, int R) {
   return C >= 1 && C <= PAIR_MOST && R >= 1 &&
-         8ll * C * C * R + 4ll * 4 * 64 * ((3 * C) | 1) <= 200ll << 10;
+         8ll * C * C * R + 4ll * 4 * 64 * ((3 * C) | 1) <= PAIR_SMEM;
 }
 
 extern "C" int ngs_basis_pairs(const ngs_basis_pair_term* p, int grad, ngs_stream s) {
@@ -447,10 +452,10 @@ extern "C" int ngs_basis_divergence(const ngs_basis_div_term* p, int grad, ngs_s
   a.mul = p->mul, a.add = p->add, a.scale = p->scale;
   a.b = p->b, a.lam = p->lam, a.gcoef = p->gcoef, a.gdata = p->gdata;
   const unsigned grid = ngs_blocks(a.pairs, 128, 8);
-  const size_t smem = sizeof(float) * 4 * 32 * ((3 * a.C) | 1);               // at most 49,664 bytes
+  const size_t smem = sizeof(float) * 4 * 32 * ((3 * a.C) | 1);               // at most ROWS_SMEM
   ngs_count_launch();
   if (grad) {
-    if (smem > 48 << 10) cudaFuncSetAttribute(basis_divergence_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 << 10) cudaFuncSetAttribute(basis_divergence_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM);
     basis_divergence_kernel<true><<<grid, 128, smem, (cudaStream_t)s>>>(a);
   } else {
     basis_divergence_kernel<false><<<grid, 128, 0, (cudaStream_t)s>>>(a);
@@ -503,7 +508,7 @@ extern "C" int ngs_basis_phi_grad(const ngs_basis_comps* comps, const float* coe
   if (!coef || !rows || !local || !lam || !xs || !pa || !pb || !gcoef) return NGS_ERR_INVALID_ARG;
   const int64_t m = 27 * n_points;
   const size_t smem = sizeof(float) * 4 * 32 * ((3 * c.count) | 1);
-  if (smem > 48 << 10) cudaFuncSetAttribute(basis_phi_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 << 10) cudaFuncSetAttribute(basis_phi_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM);
   { ngs_count_launch(); basis_phi_grad_kernel<<<ngs_blocks(m, 128, 8), 128, smem, (cudaStream_t)s>>>(c, coef, rows, local, m, lam, xs, pa, pb,
                                                                                         gcoef); }
   NGS_CHECK_LAUNCH();
