@@ -24,12 +24,12 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include "conv_plan.h"
 #include "conv_ring.h"
 #include "ngs_common.cuh"
 
 namespace conv {
 
-constexpr int BM = 128;              // tile rows (UMMA M)
 constexpr int BK = 64;               // reduction elements per stage (128 bytes of 16-bit values)
 constexpr int UK = 16;               // UMMA K of kind::f16
 constexpr int PRODUCERS = 256;       // warps 0-7
@@ -222,7 +222,6 @@ struct TileShape {
   uint32_t stage_bytes;
 };
 
-constexpr uint32_t A_BYTES = BM * 128;   // 16 KB
 constexpr int AHEAD = 2;
 
 template <bool ASYNC, typename Fill, typename Store>
@@ -234,7 +233,7 @@ NGS_DEV void run_tile(const TileShape& t, uint8_t* smem, Fill& fill, Store& stor
   __shared__ int ksteps_of[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int S = t.stages;
-  const uint32_t ncols_alloc = t.n <= 32 ? 32u : t.n <= 64 ? 64u : t.n <= 128 ? 128u : 256u;
+  const uint32_t ncols_alloc = tmem_columns(t.n);
   if (tid == 0) {
     for (int s = 0; s < S; s++) {
       mbar_init(&full_bar[s], PRODUCERS / 32);
@@ -379,7 +378,6 @@ NGS_DEV void st16_row(void* out, bool f32, int bf16, int64_t off, const float (&
 namespace conv {
 
 constexpr int TMA_THREADS = 224;         // warps 0 and 6: TMA, warp 1: MMAs, warps 2-5: cp.async, then epilogue
-constexpr int TMA_STAGES = 8;            // of the ring, at most
 
 NGS_DEV void mbar_expect(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
@@ -417,7 +415,7 @@ NGS_DEV void run_tile_tma(const TmaShape& t, uint8_t* smem, Setup& setup, Next& 
   __shared__ int ksteps_of[TMA_STAGES];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int S = t.stages;
-  const uint32_t ncols_alloc = t.n <= 32 ? 32u : t.n <= 64 ? 64u : t.n <= 128 ? 128u : 256u;
+  const uint32_t ncols_alloc = tmem_columns(t.n);
   if (tid == 0) {
     for (int s = 0; s < S; s++) {
       mbar_init(&full_bar[s], 6);
@@ -570,10 +568,9 @@ struct GatherGemm {
   int32_t oob;
 };
 
-// Rows of a tile that are copied with cp.async (a multiple of 16), and the blocks an SM is to hold.  1.3M rows of
-// 64 -> 64 channels: 776, 767 and 800 us with 32, 48 and 64 rows; 907 with three blocks.
+// Rows of a tile that are copied with cp.async (a multiple of 16).  1.3M rows of 64 -> 64 channels: 776, 767 and 800 us
+// with 32, 48 and 64 rows.
 constexpr int CP_ROWS = 48, TMA_ROWS = conv::BM - CP_ROWS;
-constexpr int CONV_PER_SM = 4;
 
 __global__ void __launch_bounds__(conv::TMA_THREADS) conv_gather_gemm_kernel(const __grid_constant__ GatherGemm g,
                                                                             const __grid_constant__ CUtensorMap xmap,
@@ -1226,20 +1223,14 @@ static int conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_
     return simt_gemm<__half>(g, st);
   }
   g.oob = n_src < 0x7fffffff ? (int32_t)std::max<int64_t>(n_src, 1) : -1;
-  // as many blocks on an SM as its shared memory and the tensor memory hold, up to CONV_PER_SM, of two stages or more
-  const size_t fixed = 1024;                                    // alignment of the first stage
-  g.stage_bytes = conv::A_BYTES + (uint32_t)((box * 128 + 1023) & ~1023);
-  for (int per_sm = std::min(CONV_PER_SM, 512 / std::max(box, 32)); per_sm >= 1; per_sm--) {
-    const size_t room = (227 << 10) / per_sm - 1536;            // the kernel's static arrays, the block's reserve
-    g.stages = fixed < room ? (int)std::min<size_t>((room - fixed) / g.stage_bytes, conv::TMA_STAGES) : 0;
-    if (g.stages >= 2) break;
-  }
-  const size_t smem = fixed + (size_t)g.stages * g.stage_bytes;
+  const conv::GatherPlan plan = conv::gather_plan(box);
+  g.stages = plan.stages;
+  g.stage_bytes = plan.stage_bytes;
   if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
     return ngs_set_cuda_error(cudaGetLastError());
   const dim3 grid((unsigned)((n_rows + conv::BM - 1) / conv::BM), (unsigned)((ncols + 255) / 256));
   ngs_count_launch();
-  conv_gather_gemm_kernel<<<grid, conv::TMA_THREADS, smem, st>>>(g, xmap, bmap);
+  conv_gather_gemm_kernel<<<grid, conv::TMA_THREADS, plan.smem, st>>>(g, xmap, bmap);
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }

@@ -213,10 +213,9 @@ def solve_cusparse(Ap, Aj, Ax, b, tol: float):
     if rowptr.shape != (n + 1,) or cols.numel() != ax64.numel():
         raise ValueError(f"CSR of {rowptr.numel() - 1} rows, {cols.numel()} columns and {ax64.numel()} values for {n} unknowns")
     if n > 0:
-        counts = rowptr[1:] - rowptr[:-1]
-        total, least = torch.stack([counts.sum(), counts.min()]).tolist()
-        if total != cols.numel() or least < 0:
-            raise ValueError(f"row pointers of {total} entries (smallest row {least}) for {cols.numel()} columns")
+        first, last, least = torch.stack([rowptr[0], rowptr[-1], (rowptr[1:] - rowptr[:-1]).min()]).tolist()
+        if first != 0 or last != cols.numel() or least < 0:
+            raise ValueError(f"row pointers from {first} to {last} (smallest row {least}) for {cols.numel()} columns")
     inv_diag = torch.empty(n, dtype=torch.float32, device=b.device)
     L.call("ngs_csr_diag_inv", L.ptr(rowptr), L.ptr(cols), L.ptr(ax64), n, L.ptr(inv_diag), L.stream())
     x, _ = _pcg(rowptr, cols, Ax, b, inv_diag, 1e-12, -1, False, L.PCG_FP64, b64=b.double(), ax64=ax64)
