@@ -947,6 +947,29 @@ __global__ void __launch_bounds__(BM* BN / 16) conv_gather_gemm_simt_kernel(
   }
 }
 
+// One thread per output, for layers too small to fill the tiles' pipeline: the same multiply-adds in the same order (a
+// missing row is skipped instead of added as zeros).
+template <typename T>
+__global__ void conv_gather_gemm_thread_kernel(const T* __restrict__ x, int64_t n_src, int kdim,
+                                               const int32_t* __restrict__ table, int64_t row_stride, int64_t k_stride,
+                                               int64_t n_rows, int K, const T* __restrict__ bt, int ncols, void* out,
+                                               int out_f32) {
+  const int64_t total = n_rows * ncols;
+  for (int64_t e = ngs_gtid(); e < total; e += ngs_gstride()) {
+    const int64_t r = e / ncols;
+    const int n = (int)(e - r * ncols);
+    float acc = 0.f;
+    for (int k = 0; k < K; k++) {
+      const int32_t src = table[r * row_stride + k * k_stride];
+      if (src < 0 || src >= n_src) continue;
+      const T* xr = x + (int64_t)src * kdim;
+      const T* br = bt + ((int64_t)k * ncols + n) * kdim;
+      for (int c = 0; c < kdim; c++) acc = fmaf(to_f(xr[c]), to_f(br[c]), acc);
+    }
+    put<T>(out, e, acc, out_f32 != 0);
+  }
+}
+
 // Weight gradient: per offset a BM x BN tile of channels, the offset's pairs split over blockIdx.x (a
 // partial per split, added in split order by conv_wgrad_reduce_kernel), a stage of 64 pairs in shared
 // memory.  Tiles smaller than 128 threads' work are kept by several groups of threads, each on its share
@@ -1119,6 +1142,14 @@ int simt_gemm_tile(const GatherGemm& g, cudaStream_t st) {
 
 template <typename T>
 int simt_gemm(const GatherGemm& g, cudaStream_t st) {
+  if (conv::simt_by_thread(g.n_rows, g.kdim, g.ncols, sizeof(T))) {
+    ngs_count_launch();
+    conv_gather_gemm_thread_kernel<T><<<ngs_blocks(g.n_rows * g.ncols, 256), 256, 0, st>>>(
+        reinterpret_cast<const T*>(g.x), g.n_src, g.kdim, g.table, g.row_stride, g.k_stride, g.n_rows, g.K,
+        reinterpret_cast<const T*>(g.bt), g.ncols, g.out, g.out_f32);
+    NGS_CHECK_LAUNCH();
+    return NGS_OK;
+  }
   if (g.ncols <= 16) return simt_gemm_tile<T, 64, 16>(g, st);
   if (g.ncols <= 32) return simt_gemm_tile<T, 64, 32>(g, st);
   return simt_gemm_tile<T, 64, 64>(g, st);

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <numeric>
 
 namespace conv {
 
@@ -35,6 +36,32 @@ inline GatherPlan gather_plan(int box) {
   }
   p.smem = fixed + (size_t)p.stages * p.stage_bytes;
   return p;
+}
+
+// Whether a gather GEMM on the CUDA cores is faster with a thread per output than in tiles of 64 rows: where there is
+// too little of it to fill the tiles' stages, one after another for every offset and 16 channels.  An estimate of both,
+// in ns per kernel offset, fitted to 1,309 layers (FP32 and 16-bit, 200 to 200,000 rows, 1 to 256 channels in and out):
+// - tiles: 1,350 a 16 channels while an SM's blocks are few, and 1.1 for 1,000 outputs (of columns padded to the tile's);
+// - a thread per output: the longer of a thread's own chain and of what the SMs issue for all of them.  A warp's lanes
+//   read rows of weights and of features, `conflicts` of them one after another: what lies in one bank, or a third of
+//   the lines they touch.
+// The choice takes at most 1.25 times what a thread per output takes, and at most 1.4 times the better one's time in all
+// but one of them (1.6).  16 -> 32 channels FP32, 1,000 rows: 24 us by thread, 35 in tiles; 8,000 rows: 138 and 36.
+// 144 -> 4 channels in 16 bits, 3,000 rows: 88 and 405.
+inline bool simt_by_thread(int64_t rows, int kdim, int ncols, int elem_bytes) {
+  const double outputs = (double)rows * ncols;
+  const double bank = std::max(1, std::gcd(kdim * elem_bytes, 128) / 4);       // a power of two up to 32
+  const double lines = std::min(1.0, kdim * elem_bytes / 128.0) / 3;           // of a row
+  const double of_weights = std::max(1.0, std::min(ncols, 32) * std::max(bank / 32, lines));
+  const double of_rows = std::max(1.0, 32.0 / ncols * std::max(bank / 32, lines));
+  const double conflicts = ncols >= 32 ? of_weights + 1 : of_weights + of_rows + 3;
+  const double work = std::max(24 + 1.5 * kdim, kdim * conflicts);
+  constexpr double WAVE = 148 * 256;                                           // a block of 256 threads to every SM
+  const double waves = (double)((int64_t)((outputs + WAVE - 1) / WAVE));
+  const double by_thread = std::max(350 + 2.9 * work, waves * WAVE * work * 6.7e-5);
+  const int padded = ncols <= 16 ? 16 : ncols <= 32 ? 32 : (ncols + 63) / 64 * 64;
+  const double tiles = (kdim + 15) / 16 * (1350 + (double)rows * padded * 1.1e-3);
+  return by_thread < tiles;
 }
 
 }  // namespace conv
