@@ -568,10 +568,12 @@ struct GatherGemm {
   int32_t oob;
 };
 
-// Rows of a tile that are copied with cp.async (a multiple of 16).  1.3M rows of 64 -> 64 channels: 776, 767 and 800 us
-// with 32, 48 and 64 rows.
-constexpr int CP_ROWS = 48, TMA_ROWS = conv::BM - CP_ROWS;
-
+// CP: rows of a tile that are copied with cp.async (a multiple of 16), the others by TMA.  48: 1.3M rows of 64 -> 64
+// channels 776, 767 and 800 us with 32, 48 and 64 rows.  TMA gathers rows of an odd number of 16-byte pieces (8 channels
+// more than a multiple of 16) at a fraction of its rate: these take 64, and 96 where an SM has more than one tile.
+// 300,000 rows, us with 48 / 64 / 96 / 128 rows: 8 -> 16 channels 305 / 247 / 162 / 182, 72 -> 128 channels 544 / 479
+// / 406 / 466; 10,000 rows: 28 / 26 / 26 / 31 and 53 / 48 / 56 / 65.
+template <int CP>
 __global__ void __launch_bounds__(conv::TMA_THREADS) conv_gather_gemm_kernel(const __grid_constant__ GatherGemm g,
                                                                             const __grid_constant__ CUtensorMap xmap,
                                                                             const __grid_constant__ CUtensorMap bmap) {
@@ -582,7 +584,8 @@ __global__ void __launch_bounds__(conv::TMA_THREADS) conv_gather_gemm_kernel(con
   const int64_t r0 = (int64_t)blockIdx.x * BM;
   const int n0 = blockIdx.y * 256, rows = (int)min((int64_t)BM, g.n_rows - r0);
   const unsigned n_src = (unsigned)g.n_src;
-  const uint32_t half = TMA_ROWS / 8 * 512;
+  constexpr int TMA_ROWS = BM - CP;
+  constexpr uint32_t half = TMA_ROWS / 8 * 512;         // bytes of a TMA warp's gathers
   TmaShape t{min(256, g.ncols - n0), g.stages, g.stage_bytes, {half + (uint32_t)min(256, g.ncols) * 128u, half}, false};
 
   // entries of rows 4 lane .. 4 lane + 3 at an offset: `oob`, a row out of the map's range (zeros), for missing ones
@@ -629,9 +632,9 @@ __global__ void __launch_bounds__(conv::TMA_THREADS) conv_gather_gemm_kernel(con
   // eight lanes per row, one 16-byte piece each
   auto copy = [&](uint8_t* a, int w) {
     const uint32_t sa = smem_u32(a);
-    const int piece = lane & 7, of4 = lane >> 3, e = c0 + piece * 8, quad0 = (TMA_ROWS + w * (CP_ROWS / 4)) / 4;
+    const int piece = lane & 7, of4 = lane >> 3, e = c0 + piece * 8, quad0 = (TMA_ROWS + w * (CP / 4)) / 4;
 #pragma unroll
-    for (int j = 0; j < CP_ROWS / 16; j++) {
+    for (int j = 0; j < CP / 16; j++) {
       const int x = __shfl_sync(0xffffffffu, src.x, quad0 + j), y = __shfl_sync(0xffffffffu, src.y, quad0 + j);
       const int z = __shfl_sync(0xffffffffu, src.z, quad0 + j), u = __shfl_sync(0xffffffffu, src.w, quad0 + j);
       const int32_t v = of4 < 2 ? (of4 == 0 ? x : y) : (of4 == 2 ? z : u);
@@ -1257,11 +1260,13 @@ static int conv_gather_gemm(const void* x, int64_t n_src, int kdim, const int32_
   const conv::GatherPlan plan = conv::gather_plan(box);
   g.stages = plan.stages;
   g.stage_bytes = plan.stage_bytes;
-  if (cudaFuncSetAttribute(conv_gather_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
+  const auto kernel = kdim % 16 == 0 ? conv_gather_gemm_kernel<48>
+                      : n_rows <= (int64_t)ngs_num_sms() * conv::BM ? conv_gather_gemm_kernel<64> : conv_gather_gemm_kernel<96>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
     return ngs_set_cuda_error(cudaGetLastError());
   const dim3 grid((unsigned)((n_rows + conv::BM - 1) / conv::BM), (unsigned)((ncols + 255) / 256));
   ngs_count_launch();
-  conv_gather_gemm_kernel<<<grid, conv::TMA_THREADS, plan.smem, st>>>(g, xmap, bmap);
+  kernel<<<grid, conv::TMA_THREADS, plan.smem, st>>>(g, xmap, bmap);
   NGS_CHECK_LAUNCH();
   return NGS_OK;
 }
