@@ -494,6 +494,9 @@ int ngs_conv_gather_gemm_kmajor(const void* x, int64_t n_src, int kdim, const in
                                 const void* bt, int ncols, int dtype, void* out, int out_f32, int* error_dev,
                                 ngs_stream s);
 size_t ngs_conv_weight_grad_ws_bytes(int K, int cin, int cout, int64_t max_pairs);
+/* The bytes that features of a type make use of: no more than above for channels that the tensor cores take; the
+ * others run with any workspace or none, the faster the more of these bytes it has. */
+size_t ngs_conv_weight_grad_ws_bytes_of(int K, int cin, int cout, int64_t max_pairs, int dtype);
 int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const void* gy, int64_t n_out, int cout,
                          const int32_t* nbmaps, const int64_t* starts_dev, int K, int64_t max_pairs, int in_col,
                          int dtype, void* grad_w, int out_f32, void* ws, size_t ws_bytes, int* error_dev, ngs_stream s);

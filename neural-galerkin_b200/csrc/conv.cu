@@ -1158,11 +1158,26 @@ int simt_gemm(const GatherGemm& g, cudaStream_t st) {
   return simt_gemm_tile<T, 64, 64>(g, st);
 }
 
-// Splits of the pairs: at least 512 pairs each (CUDA cores) or 2,048 (tensor cores), at most 64.
+// Splits of an offset's pairs, each with a partial result in the workspace: of at least `least` pairs each, at most 64.
 int wgrad_splits(int64_t max_pairs, int64_t least) {
   const int64_t s = (max_pairs + least - 1) / least;
   return (int)(s < 1 ? 1 : (s > 64 ? 64 : s));
 }
+
+// On the tensor cores splits of 2,048 pairs; on the CUDA cores of 512 while offsets, channel tiles and splits together
+// are no more than SIMT_BLOCKS, some 16 blocks an SM: more of them add partials to write and to read, not blocks that
+// run.
+constexpr int SIMT_BLOCKS = 2400;
+
+int simt_tile(int channels) { return channels <= 16 ? 16 : channels <= 32 ? 32 : 64; }
+
+int simt_splits(int K, int cin, int cout, int64_t max_pairs) {
+  const int bm = simt_tile(cin), bn = simt_tile(cout);
+  const int64_t tiles = (int64_t)K * ((cin + bm - 1) / bm) * ((cout + bn - 1) / bn);
+  return (int)std::min<int64_t>(wgrad_splits(max_pairs, 512), (SIMT_BLOCKS + tiles - 1) / tiles);
+}
+
+bool wgrad_tensor_cores(int cout, int dtype) { return (dtype == NGS_F16 || dtype == NGS_BF16) && cout % 16 == 0; }
 
 template <typename T, int BM, int BN>
 void simt_wgrad_tile(const void* x, const void* gy, int64_t n_in, int64_t n_out, int cin, int cout,
@@ -1179,21 +1194,21 @@ template <typename T>
 int simt_wgrad(const void* x, const void* gy, int64_t n_in, int64_t n_out, int cin, int cout, const int32_t* nbmaps,
                const int64_t* starts, int in_col, int K, int64_t max_pairs, void* out, int out_f32, void* ws,
                size_t ws_bytes, cudaStream_t st) {
-  // without a workspace for the partials, one split per offset
-  int splits = wgrad_splits(max_pairs, 512);
-  if (!ws || ws_bytes < (size_t)K * splits * cin * cout * sizeof(float) || !aligned16(ws)) splits = 1;
+  // as many splits as the workspace holds partials for, one (written in place) without a workspace
+  const size_t one = (size_t)K * cin * cout * sizeof(float);
+  const int splits = ws && aligned16(ws) ? (int)std::max<size_t>(1, std::min<size_t>(simt_splits(K, cin, cout, max_pairs), ws_bytes / one)) : 1;
   float* part = splits > 1 ? static_cast<float*>(ws) : nullptr;
   auto go = [&](auto bm, auto bn) {
     simt_wgrad_tile<T, decltype(bm)::value, decltype(bn)::value>(x, gy, n_in, n_out, cin, cout, nbmaps, starts, in_col,
                                                                  K, splits, part, out, out_f32, st);
   };
   auto with_bm = [&](auto bm) {
-    if (cout <= 16) go(bm, std::integral_constant<int, 16>{});
-    else if (cout <= 32) go(bm, std::integral_constant<int, 32>{});
+    if (simt_tile(cout) == 16) go(bm, std::integral_constant<int, 16>{});
+    else if (simt_tile(cout) == 32) go(bm, std::integral_constant<int, 32>{});
     else go(bm, std::integral_constant<int, 64>{});
   };
-  if (cin <= 16) with_bm(std::integral_constant<int, 16>{});
-  else if (cin <= 32) with_bm(std::integral_constant<int, 32>{});
+  if (simt_tile(cin) == 16) with_bm(std::integral_constant<int, 16>{});
+  else if (simt_tile(cin) == 32) with_bm(std::integral_constant<int, 32>{});
   else with_bm(std::integral_constant<int, 64>{});
   NGS_CHECK_LAUNCH();
   if (part) {
@@ -1286,7 +1301,13 @@ extern "C" int ngs_conv_gather_gemm_kmajor(const void* x, int64_t n_src, int kdi
 }
 
 extern "C" size_t ngs_conv_weight_grad_ws_bytes(int K, int cin, int cout, int64_t max_pairs) {
-  return (size_t)K * wgrad_splits(max_pairs, 512) * cin * cout * sizeof(float);
+  return (size_t)K * wgrad_splits(max_pairs, 2048) * cin * cout * sizeof(float);
+}
+
+extern "C" size_t ngs_conv_weight_grad_ws_bytes_of(int K, int cin, int cout, int64_t max_pairs, int dtype) {
+  if (K < 1 || cin < 1 || cout < 1 || max_pairs < 0) return 0;
+  const int splits = wgrad_tensor_cores(cout, dtype) ? wgrad_splits(max_pairs, 2048) : simt_splits(K, cin, cout, max_pairs);
+  return (size_t)K * splits * cin * cout * sizeof(float);
 }
 
 extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const void* gy, int64_t n_out, int cout,
@@ -1298,8 +1319,7 @@ extern "C" int ngs_conv_weight_grad(const void* x, int64_t n_in, int cin, const 
       (max_pairs > 0 && !nbmaps) || (n_in > 0 && !x) || (n_out > 0 && !gy))
     return NGS_ERR_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)s;
-  const bool tc = (dtype == NGS_F16 || dtype == NGS_BF16) && cout % 16 == 0 && aligned16(grad_w);
-  if (!tc) {
+  if (!wgrad_tensor_cores(cout, dtype) || !aligned16(grad_w)) {
     if (dtype == NGS_F32)
       return simt_wgrad<float>(x, gy, n_in, n_out, cin, cout, nbmaps, starts_dev, in_col, K, max_pairs, grad_w, 1, ws,
                                ws_bytes, st);

@@ -169,6 +169,7 @@ _SIGS = {
     "ngs_conv_gather_gemm": ([vp, i64, C.c_int, vp, i64, C.c_int, vp, C.c_int, C.c_int, vp, C.c_int, vp, vp],
                              C.c_int),
     "ngs_conv_weight_grad_ws_bytes": ([C.c_int, C.c_int, C.c_int, i64], sz),
+    "ngs_conv_weight_grad_ws_bytes_of": ([C.c_int, C.c_int, C.c_int, i64, C.c_int], sz),
     "ngs_conv_weight_grad": ([vp, i64, C.c_int, vp, i64, C.c_int, vp, vp, C.c_int, i64, C.c_int, C.c_int, vp,
                               C.c_int, vp, sz, vp, vp], C.c_int),
     "ngs_pcg_workspace_bytes": ([i64, C.c_int], sz),

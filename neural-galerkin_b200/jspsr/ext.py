@@ -380,7 +380,7 @@ def convolution_backward_cuda(in_feat, grad_in_feat, grad_out_feat, kernel, grad
     dt = _conv_dtype(x)
     gk = grad_kernel if (grad_kernel.is_contiguous() and grad_kernel.dtype == x.dtype) else \
         torch.empty(kernel.shape, dtype=x.dtype, device=x.device)
-    ws_bytes = L.load().ngs_conv_weight_grad_ws_bytes(K, cin, cout, max_pairs)
+    ws_bytes = L.load().ngs_conv_weight_grad_ws_bytes_of(K, cin, cout, max_pairs, dt)
     ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=x.device)
     L.call("ngs_conv_weight_grad", L.ptr(x), x.shape[0], cin, L.ptr(gy), gy.shape[0], cout, L.ptr(nbmap), L.ptr(starts),
            K, max_pairs, in_col, dt, L.ptr(gk), int(gk.dtype == torch.float32), L.ptr(ws), ws.numel(), L.ptr(err),
