@@ -227,6 +227,9 @@ class DualMesher:
                 else:
                     L.call("ngs_dual_mc_indices_grid", dg, L.ptr(epb[starts[d]:]), counts[d], self.levels[d].stride,
                            d, int(starts[d]), L.ptr(acc), 1, L.ptr(cnt), st)
+        elif np.any(dims >= (1 << 21)):
+            # what the packed corner keys hold, on either of the routes below
+            raise ValueError(f"mesh domain of {dims.tolist()} cells exceeds 2^21 cells per axis")
         elif int(dims[0]) * int(dims[1]) * ((int(dims[2]) + 4095) // 4096) <= self.dual_grid2_max_words:
             # deep hierarchies: the coarse cells stretch the box far beyond the surface, so only the
             # 64-cell words that hold a centre get one (a 5M-point room of 11 levels: 502 -> 277 ms a
@@ -235,8 +238,6 @@ class DualMesher:
         else:
             # boxes too large for that: the dual centres are de-duplicated by a sort of packed corner
             # keys and found through the key table (the reference's own route, reconstructor.py:347-357)
-            if np.any(dims >= (1 << 21)):
-                raise ValueError(f"mesh domain of {dims.tolist()} cells exceeds 2^21 cells per axis")
             nd, table = self._dual_centres_by_sort(epb, starts, counts, max_depth, lo, offs)
             acc = torch.zeros((nd, 8), dtype=torch.int32, device=dev)
             cnt = torch.zeros(nd, dtype=torch.int32, device=dev)
