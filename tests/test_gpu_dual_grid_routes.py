@@ -71,3 +71,22 @@ def test_boxes_of_2_21_cells_an_axis_are_refused(axis, two):
     cells[1, axis] = 1 << 20
     with pytest.raises(ValueError, match="2\\^21"):
         m.mesh_from_leaves({0: cells}, 1, 2, lambda p: torch.sin(p.sum(1)))
+
+
+@pytest.mark.parametrize("cells,apart,route", [(500, 4200, "sorted_keys"), (500, 3000, "two_level"), (60000, 4200, "two_level")])
+def test_route_follows_the_cells_in_the_box(cells, apart, route, taken):
+    """Two clusters of cells far apart: an outer grid of 18 or 9 million words, for few cells or for many."""
+    from jspsr.core.pipeline import DualMesher
+    g = torch.Generator(device=DEV).manual_seed(cells)
+    c = torch.unique(torch.randint(0, 60, (cells, 3), generator=g, device=DEV), dim=0)
+    c = torch.unique(torch.cat([c, c + apart // 2]), dim=0).int()
+    out = []
+    for two in (1 << 27, 0):
+        m = DualMesher()
+        m.levels = [SimpleNamespace(stride=1)]
+        m.vs, m.dev, m.dual_grid_max_words, m.dual_grid2_max_words = 1.0 / 64, DEV, 0, two
+        v, f = m.mesh_from_leaves({0: c}, 1, 2, lambda p: torch.sin(97.0 * p.sum(1) + 1.0))
+        out.append((m.mesh_info["cnt"], m.mesh_info["acc_ids"], f, v))
+    assert taken == [route, "sorted_keys"]
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
