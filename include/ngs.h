@@ -246,9 +246,9 @@ int ngs_screen_gram(const int32_t* rows, const float* phi, int64_t n, const floa
                     const int64_t* rowptr, double scale, double* vals, ngs_stream s);
 /* ngs_screen_gram with the points grouped by cell: order = the point ids sorted by keys (keys[i] is
  * the key of point order[i]: first present row of the point's 27 * 27 + that row's position, or -1
- * for a point with no voxel at this level).  One atomic per (cell chunk of at most 128 points, row,
- * column) instead of per point; the same sums up to the order of FP64 additions.  No counterpart in
- * the reference. */
+ * for a point with no voxel at this level).  One atomic per (run of a cell's points within a warp's
+ * share of at most 128, row, column) instead of per point; the same sums up to the order of FP64
+ * additions.  No counterpart in the reference. */
 /* keys[p] = first present row of rows[p, 0..26] * 27 + its position, or -1 (the cell key of
  * ngs_screen_gram_grouped). */
 int ngs_point_cell_keys(const int32_t* rows, int64_t n, int64_t* keys, ngs_stream s);
@@ -260,7 +260,7 @@ int ngs_screen_rhs(const int32_t* rows, const float* phi, int64_t n, const float
                    ngs_stream s);
 /* rhs[row] += scale * sum_p w[p] * phi[p,k] * field[p] (field nullable: 1) with the points grouped
  * by cell as for ngs_screen_gram_grouped (order / keys): one atomic per (run of a cell's points
- * within 32 sorted positions, row).  Covers ngs_screen_rhs (field NULL) and ngs_correction_screen
+ * within a warp's share of at most 256, row).  Covers ngs_screen_rhs (field NULL) and ngs_correction_screen
  * (field given, scale negated). */
 int ngs_screen_rhs_grouped(const int32_t* rows, const float* phi, int64_t n, const float* w, const float* field,
                            const int64_t* order, const int64_t* keys, double scale, double* rhs, ngs_stream s);

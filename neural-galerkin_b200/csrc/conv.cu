@@ -373,8 +373,8 @@ NGS_DEV void st16_row(void* out, bool f32, int bf16, int64_t off, const float (&
 // and the four warps of the epilogue copy the tile's last rows with cp.async meanwhile.  Both ways of copying have a
 // rate of their own.  1.3M rows of 64 -> 64 channels, 27 offsets: 1,310 us with cp.async alone (the producers'
 // instructions, 270 a step and warp), 1,128 with one warp issuing all rows by TMA (50 cycles a gather), 772 with four,
-// 760 in this form.  What is left is the chain of a step through its barriers (620 us of it remain with no bytes
-// moved at all); L2 runs at 30 % and DRAM at 7 % of their rates.
+// 760 in this form.  What is left are issue slots (70 % busy) and the steps' waits for one another, not bytes: L2 runs at
+// 31 % and DRAM at 7 % of their rates.
 namespace conv {
 
 constexpr int TMA_THREADS = 224;         // warps 0 and 6: TMA, warp 1: MMAs, warps 2-5: cp.async, then epilogue
@@ -403,7 +403,6 @@ NGS_DEV void tma_tile(uint32_t dst, const CUtensorMap* map, int c, int r, uint64
 struct TmaShape {
   int n, stages;
   uint32_t stage_bytes, tx[2];
-  bool mn_major;
 };
 
 template <typename Setup, typename Next, typename Issue, typename Copy, typename Store>
@@ -482,7 +481,7 @@ NGS_DEV void run_tile_tma(const TmaShape& t, uint8_t* smem, Setup& setup, Next& 
     cp_async_wait<0>();
     if (last >= 0) hand_over(last);
   } else if (warp == 1 && lane == 0) {
-    const uint32_t idesc = t.mn_major ? f16_idesc_mn(BM, t.n, bf16) : f16_idesc(BM, t.n, bf16);
+    const uint32_t idesc = f16_idesc(BM, t.n, bf16);
     int st = 0;
     uint32_t parity = 0u, accumulate = 0u;
     for (;;) {
@@ -492,8 +491,7 @@ NGS_DEV void run_tile_tma(const TmaShape& t, uint8_t* smem, Setup& setup, Next& 
       const int ks = ksteps_of[st];
       if (ks == 0) break;
       for (int kk = 0; kk < ks; kk++) {
-        umma_f16(tmem, t.mn_major ? mnmajor_sw128_desc(a + kk * 2048) : kmajor_sw128_desc(a + kk * 32),
-                 t.mn_major ? mnmajor_sw128_desc(b + kk * 2048) : kmajor_sw128_desc(b + kk * 32), idesc, accumulate);
+        umma_f16(tmem, kmajor_sw128_desc(a + kk * 32), kmajor_sw128_desc(b + kk * 32), idesc, accumulate);
         accumulate = 1u;
       }
       umma_commit(&empty_bar[st]);
@@ -586,7 +584,7 @@ __global__ void __launch_bounds__(conv::TMA_THREADS) conv_gather_gemm_kernel(con
   const unsigned n_src = (unsigned)g.n_src;
   constexpr int TMA_ROWS = BM - CP;
   constexpr uint32_t half = TMA_ROWS / 8 * 512;         // bytes of a TMA warp's gathers
-  TmaShape t{min(256, g.ncols - n0), g.stages, g.stage_bytes, {half + (uint32_t)min(256, g.ncols) * 128u, half}, false};
+  TmaShape t{min(256, g.ncols - n0), g.stages, g.stage_bytes, {half + (uint32_t)min(256, g.ncols) * 128u, half}};
 
   // entries of rows 4 lane .. 4 lane + 3 at an offset: `oob`, a row out of the map's range (zeros), for missing ones
   const int32_t* const te = g.table + (r0 + 4 * lane) * g.row_stride;

@@ -12,10 +12,10 @@
 //                          have arrived sums all partials itself in block order
 //                          (deterministic, the same bits in every block).
 // The SpMV streams the matrix straight from HBM, eight lanes per row at two blocks per SM: a packed
-// copy of it (four rows to a warp, at spmv_packed), or a caller's CSR in one of two forms -- 4-byte columns, a row at a time with up to eight (column, value) pairs
-// and their vector gathers in flight per lane, or 2-byte column deltas in a software-pipelined
-// loop that gathers from a shared-memory window of the vector -- each with its own kernel for the
-// single-system and cluster solves.  (Staging CSR tiles through shared memory with bulk copies ran
+// copy of it (four rows to a warp, at spmv_packed), or the CSR in one of two forms -- 4-byte columns, a
+// row at a time with up to eight (column, value) pairs and their vector gathers in flight per lane, or
+// 2-byte column deltas in a software-pipelined loop that gathers from a shared-memory window of the
+// vector -- each with its own kernel for the single-system and cluster solves.  (Staging CSR tiles through shared memory with bulk copies ran
 // at less than half this rate: the product and row-sum passes over shared memory, not the copies,
 // bounded it.)
 // Every wait is bounded by the global nanosecond timer; on timeout the kernel
@@ -283,11 +283,12 @@ NGS_DEV void spmv_rows_plain(const PcgArgs& a, const MT* __restrict__ vals, cons
 // entries as in the row-at-a-time form.
 //
 // Bound: latency and wavefronts of the vector's gathers (a product of the 300k-point scene's level 0 gathers
-// 74M floats, half of them from L1; DRAM runs at 3.5 of 6.5 TB/s).  So up to 16 units (12 with 4-byte columns
-// or FP64 values, whose registers would spill) are loaded together and then gathered together, and the next
-// group's lines are prefetched to L2, which holds no register.  Measured, all solves of a level, CSR form ->
-// packed: 300k points 9.19 -> 8.30 and 3.53 -> 3.17 ms, 0.93 -> 0.76, 0.42 -> 0.43; 5M-point room 90.9 -> 73.3
-// and 15.9 -> 13.5 against the packed form without the prefetch.
+// 74M floats, half of them from L1; DRAM runs at 4.7 of 6.5 TB/s).  So up to 16 units (12 with 4-byte columns
+// or FP64 values) are loaded together and then gathered together, and the next group's lines are prefetched to
+// L2, which holds no register.  Registers spill all the same with 4-byte columns (64 bytes of stores in the mixed
+// mode's kernel; batches of eight alone do not change that).  Measured, all solves of a level of the mixed mode, CSR
+// form -> packed: 300k points 9.12 -> 8.20, 3.52 -> 3.10, 0.91 -> 0.79 and 0.45 -> 0.42 ms; levels 0 to 2 of a
+// 5M-point room 91.4 -> 75.3, 15.9 -> 13.9 and 2.42 -> 2.14.
 template <bool STREAM, bool WIDE, typename MT, typename VT, typename ACC, typename Pre, typename Epi>
 NGS_DEV void spmv_packed(const PcgArgs& a, const VT* v, int64_t row0, int64_t row1, Pre pre, Epi epi, double& dsum) {
   constexpr int WARPS = PCG_THREADS / 32;
