@@ -45,9 +45,9 @@ inline GatherPlan gather_plan(int box) {
 // - a thread per output: the longer of a thread's own chain and of what the SMs issue for all of them.  A warp's lanes
 //   read rows of weights and of features, `conflicts` of them one after another: what lies in one bank, or a third of
 //   the lines they touch.
-// The choice takes at most 1.25 times what a thread per output takes, and at most 1.4 times the better one's time in all
-// but one of them (1.6).  16 -> 32 channels FP32, 1,000 rows: 24 us by thread, 35 in tiles; 8,000 rows: 138 and 36.
-// 144 -> 4 channels in 16 bits, 3,000 rows: 88 and 405.
+// The choice takes at most 1.23 times what a thread per output takes, and at most 1.4 times the better one's time in all
+// but one of them (1.53).  16 -> 32 channels FP32, 1,000 rows: 24 us by thread, 35 in tiles; 8,000 rows: 138 and 36.
+// 144 -> 4 channels in 16 bits, 3,000 rows: 92 and 405.
 inline bool simt_by_thread(int64_t rows, int kdim, int ncols, int elem_bytes) {
   const double outputs = (double)rows * ncols;
   const double bank = std::max(1, std::gcd(kdim * elem_bytes, 128) / 4);       // a power of two up to 32
